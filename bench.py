@@ -16,7 +16,7 @@ coset vector, filtered (maxRun 3, GC [0.3,0.7]) to 207,432 words, editDist 4:
                into pinned memory (wall clock around the synchronous calls).
 * roofline  -- the pair-test kernel against the ALU-pipe peak (SMs x 64
                LOP3/PRMT lanes x max SM clock); algorithmic work = the ALU-pipe
-               ops the lane recurrence issues per pair test (alu_ops_per_pair),
+               ops the bit-sliced test needs (sliced_ops_per_pair),
                measured traffic from the committed ncu summary.  The 16*L
                integer-op convention against the INT32 peak is reported beside
                it (int_ops_16L_convention).
@@ -301,9 +301,64 @@ def touched_cells(n: int, seg_width: int, segments: int, band_rows: int = 256) -
     return int(np.sum(rows * np.maximum(segments - first, 0)))
 
 
+def sliced_ops_per_pair(L: int, d: int) -> float:
+    """LOP3 operations of the bit-sliced pair test (ig_slice.cuh) per pair
+    test.  Level form (editDist <= 5): the recurrence's and/or terms as
+    three-input operations, constants folded, only what reaches the result.
+    Delta form: 5 per band cell, 4 fewer per row, plus 2 per row for the
+    distance counter (not folded)."""
+    k = d - 1
+    if k >= L:  # every pair
+        return 1 / 32
+    if k < 2:  # mismatch levels only
+        return (1 + k) * L / 32
+    w = k // 2
+    if k > 4:
+        return L * (5 * (2 * w + 1) - 4 + 2) / 32
+    nodes, one, zero = [], "one", "zero"
+
+    def op(*ins):
+        nodes.append([x for x in ins if x != "match"])
+        return len(nodes) - 1
+
+    def fold(prev, terms):  # (prev & match) | terms
+        if one in terms:
+            return one
+        rest = [t for t in terms if t != zero]
+        if prev == one:
+            acc = ["match"] + rest
+        elif prev == zero:
+            acc = rest
+        else:
+            acc = [op(prev, *rest[:1])] + rest[1:]
+        while len(acc) > 1:
+            acc = [op(*acc[:3])] + acc[3:]
+        return acc[0] if acc else zero
+
+    ok = lambda t, e: abs(t) <= w and abs(t) <= e <= k - abs(t)
+    S = {(t, e): one if 0 <= t <= e else zero for t in range(-w, w + 1) for e in range(k + 1)}
+    for i in range(1, L + 1):
+        for t in range(-w, w + 1):
+            if i + t == 0:
+                S.update({(t, e): one if e >= -t else zero for e in range(k + 1)})
+            if not 1 <= i + t <= L:
+                continue
+            for e in range(k, -1, -1):
+                if ok(t, e):
+                    S[t, e] = fold(S[t, e], [S[q] for q in ((t, e - 1), (t + 1, e - 1), (t - 1, e - 1)) if ok(*q)])
+    live, todo = set(), [S[0, k]]
+    while todo:
+        x = todo.pop()
+        if x not in live and x != "match":
+            live.add(x)
+            todo += nodes[x]
+    return len(live) / 32
+
+
 def alu_ops_per_pair(L: int, d: int) -> float:
-    """ALU-pipe operations (LOP3, PRMT, the add and the shift) the pair-test
-    recurrence issues per pair test, counted from the kernel source (the lane
+    """ALU-pipe operations (LOP3, PRMT, the add and the shift) per pair test of
+    the recurrence with one lane per pair test that the bit-sliced test
+    replaced, kept to compare rates across versions.  Counted from its source (the lane
     counter runs as an IMAD on the FMA pipe and is not counted).  Banded
     8-lane form (two rows x four columns, editDist <= 4): 11 per character
     step for 8 pairs, 5 fewer in the last step (its vertical deltas are not
@@ -918,7 +973,7 @@ def run_ours(args, wl, rank, world, dist):
     alu_peak = props.multi_processor_count * 64 * sm_mhz * 1e6 / 1e12  # ALU pipe: 64 lanes/clk/SM
     int32_peak = props.multi_processor_count * 128 * sm_mhz * 1e6 / 1e12
     pair_avg_s = (pair_ms / max(pair_launches, 1)) / 1e3
-    alu_ops = pairs * alu_ops_per_pair(L, d)
+    alu_ops = pairs * sliced_ops_per_pair(L, d)
     achieved = alu_ops / pair_avg_s / 1e12 if pair_launches else None
     conv_ops = pairs * 16 * L
     conv_achieved = conv_ops / pair_avg_s / 1e12 if pair_launches else None
@@ -941,15 +996,15 @@ def run_ours(args, wl, rank, world, dist):
         "e2e": e2e,
         "roofline": {"bound": "int32-alu-pipe", "achieved": achieved, "peak": alu_peak, "unit": "Tops/s",
                      "frac": (achieved / alu_peak) if achieved else None, "traffic": traffic,
-                     "kernel": "pair_kernel", "kernel_ms_per_launch": pair_avg_s * 1e3,
-                     "work": f"{pairs} pair tests x {alu_ops_per_pair(L, d):g} ALU-pipe ops (LOP3/PRMT/add/shift) per pair "
+                     "kernel": "pair_levels", "kernel_ms_per_launch": pair_avg_s * 1e3,
+                     "work": f"{pairs} pair tests x {sliced_ops_per_pair(L, d):g} ALU-pipe ops (LOP3, 32 pair tests each) per pair "
                              f"test per launch",
                      "peak_source": f"{props.multi_processor_count} SMs x 64 ALU-pipe lanes/clk x {sm_mhz:.0f} MHz "
                                     f"max SM clock ({src} MEASURED_PEAKS sm_max_mhz)",
                      "int_ops_16L_convention": {"ops_per_pair": 16 * L, "achieved_tops": conv_achieved,
                                            "int32_peak_tops": int32_peak,
                                            "ratio": (conv_achieved / int32_peak) if conv_achieved else None,
-                                           "note": "16*L int ops per pair test credited; the banded multi-lane "
+                                           "note": "16*L int ops per pair test credited; the bit-sliced "
                                                    "kernel does several pair tests per op, so this exceeds 1"}},
         "compaction": {"bound": "hbm", "achieved": comp_bytes / comp_avg_s / 1e9 if comp_launches else None,
                        "peak": hbm_peak, "unit": "GB/s",

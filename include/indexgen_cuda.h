@@ -85,10 +85,11 @@ ig_status ig_ctx_phase_time(const ig_ctx *ctx, int phase, double *ms, int64_t *l
  * items per CTA of the grid -- sets how many items a batch is cut into and so
  * each job's segment width (256 .. 16,384 columns): wide tiles amortise the
  * per-item setup, narrow ones even out the end of the launch.  It is kept per
- * lane form of the pair kernel, which (len, min_ed) selects: */
-#define IG_LANES_FULL 0   /* full Myers lanes (min_ed > 8)                   */
-#define IG_LANES_NIBBLE 1 /* 8 banded nibble lanes per word (min_ed <= 4)    */
-#define IG_LANES_BYTE 2   /* 4 banded byte lanes per word (5 <= min_ed <= 8) */
+ * lane form, a class of thresholds that (len, min_ed) selects (the names are
+ * those of the lane widths each class once ran with): */
+#define IG_LANES_FULL 0   /* min_ed > 8 (or < 1)  */
+#define IG_LANES_NIBBLE 1 /* 1 <= min_ed <= 4     */
+#define IG_LANES_BYTE 2   /* 5 <= min_ed <= 8     */
 /* Lane form for (len, min_ed); -1 when len is out of range. */
 int ig_lane_form(int len, int min_ed);
 /* Times the count-only pair pass of a representative job (host or device

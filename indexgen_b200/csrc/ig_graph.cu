@@ -6,19 +6,19 @@
 // Pipeline for a batch of independent jobs (one job = n words of one length L
 // and a threshold d; edge iff ED < d).  A single job is a batch of one; the
 // clustered solve (src/SparseMat.cpp:927-1095) submits all clusters at once.
-//   prep_units      words -> PRMT selector streams, two columns per unit for L <= 15
-//   pair_kernel     ONE persistent launch for the whole batch: CTAs take
-//                   (job, row band, column segment) items from an atomic queue and
-//                   dispatch on the job's L and lane form; 256 rows per band, one
-//                   per thread, keep their match masks in registers; column tiles
-//                   of the segment are staged into shared memory by cp.async.bulk
-//                   (TMA bulk copy, no multicast) with a two-slot mbarrier
-//                   pipeline; each thread tests its row against 4 (byte lanes,
-//                   editDist 5..8) or 2/1 (full Myers) columns per 32-bit word
-//                   (pair_kernel_nib: two rows against 4 columns, nibble lanes,
-//                   editDist <= 4, 128 threads per band) and emits hits as
-//                   (row, col, rank-in-(row,segment), cell) records into slots
-//                   its warp takes in chunks, plus a per-(row, segment) count.
+//   prep_units      words -> units of 64 columns: four one-hot words per
+//                   position and 32 columns (ig_slice.cuh)
+//   pair_kernel     ONE persistent launch per form for the whole batch: CTAs
+//                   take (job, row band, column segment) items from an atomic
+//                   queue and dispatch on the job's length and threshold; 256
+//                   rows per band, one per thread; column tiles of the segment
+//                   are staged into shared memory by cp.async.bulk (TMA bulk
+//                   copy, no multicast) with a two-slot mbarrier pipeline; each
+//                   thread tests its row against 64 columns at a time, bit-
+//                   sliced (pair_levels: editDist <= 5, pair_deltas: above),
+//                   and emits hits as (cell, column offset, rank) records into
+//                   slots its warp takes in chunks, plus a per-(row, segment)
+//                   count.
 //   row_prefix      per-row exclusive prefix over its segments + degree
 //   scan            exclusive scan of degrees -> row_ptr (int64)
 //   scatter         cols[row_ptr[r] + prefix[cell] + rank] = col
@@ -30,23 +30,14 @@
 #include <cstring>
 
 #include "ig_internal.h"
-#include "ig_myers.cuh"
+#include "ig_slice.cuh"
 
 namespace ig {
 
 namespace {
 
-using myers::BandConst;
-using myers::BandUnit;
-using myers::kModeByte;
-using myers::kModeFull;
-using myers::kModeNib;
-using myers::Unit;
-using myers::imad;
-using myers::myers_one;
-using myers::myers_two;
-using myers::nib;
-using myers::row_pools;
+using slice::kUnitCols;
+using slice::Words2;
 
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -139,77 +130,42 @@ __device__ __forceinline__ int find_job_by_row(const JobDesc *jobs, int njobs, l
     return lo;
 }
 
-// Column units of every job: two columns per unit (16 selector words) for
-// L <= 15, one column per unit (8 words, two positions each) for L = 16.
+// Column units of every job, one warp per unit of 64 columns: word (j, c, h)
+// has bit b set where column 32 h + b of the unit has character c at position
+// j.  A warp reads its 64 words, and each position's two character bits become
+// two ballots per 32 columns, from which lane 4 (j % 8) + c forms character
+// c's word.
 __global__ void prep_units(const uint32_t *__restrict__ words, const JobDesc *__restrict__ jobs, int njobs,
                            long long total_units, uint4 *__restrict__ units)
 {
-    const long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long u = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (u >= total_units)
         return;
-    const JobDesc J = jobs[find_job_by_unit(jobs, njobs, u)];
+    const JobDesc &J = jobs[find_job_by_unit(jobs, njobs, u)];
     const long long p = u - J.unit_start;
+    const long long c0 = p * kUnitCols;
     const uint32_t *w = words + J.word_off;
-    uint4 *out = units + J.unit_off;
-    if (J.mode == kModeNib) {
-        // 4 columns; word j: nibble l = char of column l at position j
-        uint32_t cw[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            cw[c] = (4 * p + c < J.n) ? w[4 * p + c] : 0u;
-        uint32_t o[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t x = 0u;
-#pragma unroll
-            for (int l = 0; l < 4; ++l)
-                x |= ((cw[l] >> (2 * j)) & 3u) << (4 * l);
-            o[j] = (j < J.L) ? x : 0u;
-        }
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-            out[4 * p + v] = make_uint4(o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
-        return;
-    }
-    if (J.mode == kModeByte) {
-        // 4 columns; word q: positions 2q (bits 0..15) and 2q+1 (16..31)
-        uint32_t cw[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            cw[c] = (4 * p + c < J.n) ? w[4 * p + c] : 0u;
-        uint32_t o[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            uint32_t x = 0u;
-#pragma unroll
-            for (int l = 0; l < 4; ++l) {
-                x |= ((cw[l] >> (4 * q)) & 3u) << (4 * l);
-                x |= ((cw[l] >> (4 * q + 2)) & 3u) << (16 + 4 * l);
+    const bool oka = c0 + lane < J.n, okb = c0 + 32 + lane < J.n;
+    const uint32_t wa = oka ? w[c0 + lane] : 0u;
+    const uint32_t wb = okb ? w[c0 + 32 + lane] : 0u;
+    const uint32_t va = __ballot_sync(kFull, oka), vb = __ballot_sync(kFull, okb);
+    uint2 *out = reinterpret_cast<uint2 *>(units + J.unit_off + p * slice::unit_vec(J.L));
+    const uint32_t clo = (lane & 1) ? kFull : 0u, chi = (lane & 2) ? kFull : 0u;
+    for (int j0 = 0; j0 < J.L; j0 += 8) {
+        uint2 mine = make_uint2(0u, 0u);
+        for (int j = j0; j < min(j0 + 8, J.L); ++j) {
+            const uint32_t la = __ballot_sync(kFull, (wa >> (2 * j)) & 1u);
+            const uint32_t ha = __ballot_sync(kFull, (wa >> (2 * j + 1)) & 1u);
+            const uint32_t lb = __ballot_sync(kFull, (wb >> (2 * j)) & 1u);
+            const uint32_t hb = __ballot_sync(kFull, (wb >> (2 * j + 1)) & 1u);
+            if ((lane >> 2) == j - j0) {
+                mine.x = ~((la ^ clo) | (ha ^ chi)) & va;
+                mine.y = ~((lb ^ clo) | (hb ^ chi)) & vb;
             }
-            o[q] = x;
         }
-        out[2 * p] = make_uint4(o[0], o[1], o[2], o[3]);
-        out[2 * p + 1] = make_uint4(o[4], o[5], o[6], o[7]);
-        return;
-    }
-    if (J.L <= 15) {
-        const uint32_t wa = w[2 * p];
-        const uint32_t wb = (2 * p + 1 < J.n) ? w[2 * p + 1] : wa;
-        uint32_t o[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k)
-            o[k] = (k < J.L) ? (nib((wa >> (2 * k)) & 3u) | (nib((wb >> (2 * k)) & 3u) << 8)) : 0u;
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-            out[4 * p + v] = make_uint4(o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
-    } else {
-        const uint32_t x = w[p];
-        uint32_t o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            o[j] = nib((x >> (4 * j)) & 3u) | (nib((x >> (4 * j + 2)) & 3u) << 16);
-        out[2 * p] = make_uint4(o[0], o[1], o[2], o[3]);
-        out[2 * p + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+        if (j0 + (lane >> 2) < J.L)
+            out[4 * j0 + lane] = mine;
     }
 }
 
@@ -219,11 +175,7 @@ struct PairArgs {
     const JobDesc *jobs;
     int njobs;
     long long items;
-    uint32_t one;     // 1, 2, 2^16 as opaque operands for imad / umulhi
-    uint32_t two;
-    uint32_t hi;
-    uint32_t gather;  // 0x00204081 and 16, opaque: hit flags -> column mask on the FMA pipe
-    uint32_t h4;
+    uint32_t one;     // 1, as an operand the compiler cannot see (imad)
     unsigned long long *work;
     unsigned long long *rec_count;  // record slots handed out (chunks of kSlotChunk)
     unsigned long long *hit_count;  // pair tests that are edges (exact)
@@ -236,99 +188,104 @@ struct PairArgs {
     int skip_first_copy;    // test hook: withhold the first tile copy of the kernel's first item
 };
 
+// A pair CTA's shared state.  The item functions below are calls, not inlined
+// (one per length and threshold: together in one body they cost the register
+// allocator a stack frame of 1.8 KB), so what they share is at file scope,
+// where its loads stay shared-memory loads; each kernel's thread 0 copies its
+// arguments in.
+constexpr int kTileCols = 1024;                                        // columns per staged tile
+constexpr int kSlotVec = kTileCols / kUnitCols * slice::unit_vec(IG_MAX_LEN);  // uint4 per ring slot (8 KiB)
+__shared__ __align__(128) uint4 g_tile[2][kSlotVec];
+__shared__ __align__(8) uint64_t g_bar[2];
+__shared__ PairArgs g_args;
+__shared__ long long g_item;
+
 // Record slots.  Each warp takes slots from the global counter in chunks of
 // kSlotChunk (one atomic per chunk instead of one per hit group: a single
 // counter address is otherwise the limit on dense graphs) and keeps the rest
-// of its chunk in shared memory.  Slots a warp never fills are written as
-// sentinels (cell = kNoCell) when the kernel ends; the scatter skips them.
+// of its chunk, the same in every lane's registers.  Slots a warp never fills
+// are written as sentinels (cell = kNoCell) when the kernel ends; the scatter
+// skips them.
 constexpr unsigned kSlotChunk = 64;
 constexpr uint32_t kNoCell = 0xffffffffu;
 
-// Two scalar arrays, each element read and written on its own (a 16-byte
-// struct here, read whole, faulted with a misaligned shared access).
-__shared__ unsigned long long g_slot_base[kBandRows / 32];  // next free slot of each warp's chunk
-__shared__ unsigned g_slot_left[kBandRows / 32];            // free slots left in it
+struct WarpSlots {
+    unsigned long long base;  // next free slot of the warp's chunk
+    unsigned left;            // free slots left in it
+};
 
 // Slots of the warp's next `total` records (warp-uniform call): record j goes
-// to b0 + j for j < n0, else to b1 + (j - n0).
+// to b0 + j for j < n0, else to b1 + j (b1 already less n0).
 struct Slots {
     unsigned long long b0, b1;
     unsigned n0;
 };
 
-__device__ __forceinline__ Slots take_slots(const PairArgs &a, unsigned total, int lane)
+__device__ __forceinline__ Slots take_slots(WarpSlots &w, unsigned total, int lane)
 {
-    const int w = threadIdx.x >> 5;
-    unsigned long long b0 = 0, b1 = 0;
-    unsigned n0 = 0;
-    if (lane == 0) {
-        b0 = g_slot_base[w];
-        const unsigned left = g_slot_left[w];
-        if (left >= total) {
-            n0 = total;
-            g_slot_base[w] = b0 + total;
-            g_slot_left[w] = left - total;
-        } else {
-            n0 = left;
-            const unsigned need = total - left;
-            const unsigned take = need > kSlotChunk ? need : kSlotChunk;
-            b1 = atomicAdd(a.rec_count, (unsigned long long)take);
-            g_slot_base[w] = b1 + need;
-            g_slot_left[w] = take - need;
-        }
-    }
     Slots s;
-    s.b0 = __shfl_sync(kFull, b0, 0);
-    s.b1 = __shfl_sync(kFull, b1, 0);
-    s.n0 = __shfl_sync(kFull, n0, 0);
+    s.b0 = w.base;
+    s.b1 = 0;
+    s.n0 = total;
+    if (w.left >= total) {
+        w.base += total;
+        w.left -= total;
+        return s;
+    }
+    s.n0 = w.left;
+    const unsigned need = total - w.left;
+    const unsigned take = need > kSlotChunk ? need : kSlotChunk;
+    unsigned long long b1 = 0;
+    if (lane == 0)
+        b1 = atomicAdd(g_args.rec_count, (unsigned long long)take);
+    b1 = __shfl_sync(kFull, b1, 0);
+    s.b1 = b1 - s.n0;
+    w.base = b1 + need;
+    w.left = take - need;
     return s;
 }
 
-// Hit flags at bits 7, 15, 23, 31 of h (all other bits clear) -> bits 0..3.
-// The multiply by 2^21 + 2^14 + 2^7 + 1 moves bit 8c+7 to bit 28+c and puts
-// every other partial product on a distinct bit below 28 or above 31 (no
-// carries), and the high half of a multiply by 16 is bits 28..31: two FMA-pipe
-// operations instead of seven shifts and masks on the ALU pipe.
-__device__ __forceinline__ uint32_t hit_columns(uint32_t h, const PairArgs &a)
+// Integer multiply-add with an operand the compiler cannot see as a constant,
+// so it stays an IMAD on the FMA pipe instead of an add on the ALU pipe (the
+// pipe the logic operations saturate).
+__device__ __forceinline__ uint32_t imad(uint32_t a, uint32_t b, uint32_t c)
 {
-    return __umulhi(myers::imad(h, a.gather, 0u), a.h4);
+    uint32_t d;
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
 }
 
 // Warp total of cnt and this lane's exclusive prefix.  When no lane has more
-// than one hit (the usual case on sparse graphs) one ballot gives both;
-// otherwise the bit planes of cnt (kPlanes of them) are balloted.
-template <int kPlanes>
+// than one hit (the usual case on sparse graphs) one ballot gives both,
+// otherwise a shuffle scan does.
 __device__ __forceinline__ void warp_count_prefix(uint32_t cnt, int lane, unsigned &total, unsigned &pre)
 {
-    const unsigned lt = (1u << lane) - 1u;
     const unsigned some = __ballot_sync(kFull, cnt != 0u);
     if (__all_sync(kFull, cnt <= 1u)) {
         total = (unsigned)__popc(some);
-        pre = (unsigned)__popc(some & lt);
+        pre = (unsigned)__popc(some & ((1u << lane) - 1u));
         return;
     }
-    total = 0;
-    pre = 0;
+    unsigned incl = cnt;
 #pragma unroll
-    for (int b = 0; b < kPlanes; ++b) {
-        const unsigned bal = __ballot_sync(kFull, (cnt >> b) & 1u);
-        total += (unsigned)__popc(bal) << b;
-        pre += (unsigned)__popc(bal & lt) << b;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o)
+            incl += t;
     }
+    total = __shfl_sync(kFull, incl, 31);
+    pre = incl - cnt;
 }
 
-constexpr int kSlotVec = kTileCols * 2;  // uint4 per staged tile (8 KiB, every unit layout)
-
-// Thread 0: copy the tile of units starting at column c0 (at most kTile
+// Thread 0: copy the tile of units starting at column c0 (at most kTileCols
 // columns, up to c_hi) into ring slot `slot`.
-template <int kTile, int kCols, int kVec>
-__device__ __forceinline__ void ring_issue(uint4 (*tile)[kSlotVec], uint64_t *bar, int slot, const uint4 *units,
-                                           int32_t c0, int32_t c_hi)
+template <int L>
+__device__ __forceinline__ void ring_issue(int slot, const uint4 *units, int32_t c0, int32_t c_hi)
 {
-    const int nu = (min(kTile, c_hi - c0) + kCols - 1) / kCols;
-    const uint32_t bytes = (uint32_t)nu * kVec * 16;
-    mbar_arrive_expect_tx(&bar[slot], bytes);
-    bulk_g2s(&tile[slot][0], units + (size_t)(c0 / kCols) * kVec, bytes, &bar[slot]);
+    const int nu = (min(kTileCols, c_hi - c0) + kUnitCols - 1) / kUnitCols;
+    const uint32_t bytes = (uint32_t)nu * slice::unit_vec(L) * 16;
+    mbar_arrive_expect_tx(&g_bar[slot], bytes);
+    bulk_g2s(&g_tile[slot][0], units + (size_t)(c0 / kUnitCols) * slice::unit_vec(L), bytes, &g_bar[slot]);
 }
 
 // Ring state bits: bit s (s = 0, 1) is the phase parity slot s waits for
@@ -346,9 +303,9 @@ constexpr uint32_t kSkipped = 4u;
 // slot b's copy was issued, bit 2 = the other slot's copy was issued.
 __shared__ uint32_t g_drain;
 
-__device__ __forceinline__ void ring_note_abort(const PairArgs &a, int b, bool b_issued, bool other_issued)
+__device__ __forceinline__ void ring_note_abort(int b, bool b_issued, bool other_issued)
 {
-    atomicCAS(a.status, kStatusOk, kStatusTimeout);
+    atomicCAS(g_args.status, kStatusOk, kStatusTimeout);
     g_drain = (uint32_t)b | (b_issued ? 2u : 0u) | (other_issued ? 4u : 0u);
 }
 
@@ -356,7 +313,7 @@ __device__ __forceinline__ void ring_note_abort(const PairArgs &a, int b, bool b
 // already advanced past the phase that timed out.  Waiting on a phase that
 // has completed returns at once; a copy that never lands is reported as
 // kStatusCopyLost.
-__device__ __forceinline__ void ring_drain(const PairArgs &a, uint64_t *bar, uint32_t parity)
+__device__ __forceinline__ void ring_drain(uint32_t parity)
 {
     const uint32_t d = g_drain;
     const int b = (int)(d & 1u);
@@ -365,276 +322,195 @@ __device__ __forceinline__ void ring_drain(const PairArgs &a, uint64_t *bar, uin
         if (!((d >> (slot == b ? 1 : 2)) & 1u))
             continue;
         const long long t0 = clock64();
-        while (!mbar_try_wait(&bar[slot], (pend >> slot) & 1u)) {
-            if (clock64() - t0 > a.wait_cycles) {
-                atomicExch(a.status, kStatusCopyLost);
+        while (!mbar_try_wait(&g_bar[slot], (pend >> slot) & 1u)) {
+            if (clock64() - t0 > g_args.wait_cycles) {
+                atomicExch(g_args.status, kStatusCopyLost);
                 break;
             }
         }
     }
 }
 
-// Everything one thread needs about its row while it walks a segment.
-struct RowCtx {
-    int32_t row;     // job-local row
-    bool ok;         // row < n
-    uint32_t p01, p23;
-    int32_t seg0;    // job-local first column of the segment
-    uint32_t cell;   // index of this (row, segment) count
-    int32_t n;
-    int lim;
-};
-
-// Bits [lo, hi) of the columns col0 + c, c < NC, that lie in the strict upper
-// triangle of the job (col > row, col < n) for a valid row.
-template <int NC>
-__device__ __forceinline__ uint32_t upper_mask(const RowCtx &r, int32_t col0)
+// Bits [0, 32) of the columns col0 + c that lie in the strict upper triangle
+// of the job (col > row, col < n) for a valid row.
+__device__ __forceinline__ uint32_t upper_mask(int32_t row, int32_t n, int32_t col0)
 {
-    if (!r.ok)
-        return 0u;
-    const int lo = max(r.row + 1 - col0, 0);
-    const int hi = min(r.n - col0, NC);
-    return hi > lo ? (((1u << hi) - 1u) & ~((1u << lo) - 1u)) : 0u;
+    const int lo = min(max(row + 1 - col0, 0), 32);
+    const int hi = min(max(n - col0, 0), 32);
+    const uint32_t below_lo = lo >= 32 ? kFull : (1u << lo) - 1u;
+    const uint32_t below_hi = hi >= 32 ? kFull : (1u << hi) - 1u;
+    return row < n ? below_hi & ~below_lo : 0u;
 }
 
-// Emit this thread's hits m (bit c: column col0 + c, c < NC) for a warp in
-// which at least one lane has a hit.  Ranks count the row's hits in its
-// (row, segment) cell in column order, so the scatter needs no sort.
-template <int NC>
-__device__ __forceinline__ void emit_mask(const PairArgs &a, uint32_t m, const RowCtx &r, int32_t col0,
-                                          uint32_t &rank, int lane)
+// Records of one word's hits m (bit c: column offset off0 + c in the segment)
+// at warp record numbers j, j+1, ... of the slots sl.  Ranks count the row's
+// hits in its (row, segment) cell in column order, so the scatter needs no
+// sort.
+__device__ __forceinline__ void write_hits(EdgeRecord *rec, unsigned long long cap, uint32_t m, uint32_t cell, uint32_t off0,
+                                           uint32_t &rank, const Slots &sl, unsigned &j)
 {
-    const uint32_t cnt = __popc(m);
-    if (!a.emit) {
-        rank += cnt;
-        return;
-    }
-    // warp total and this lane's exclusive prefix
-    constexpr int kPlanes = NC >= 8 ? 4 : (NC >= 4 ? 3 : (NC >= 2 ? 2 : 1));
-    unsigned total, pre;
-    warp_count_prefix<kPlanes>(cnt, lane, total, pre);
-    if (total == 0u)
-        return;
-    const Slots sl = take_slots(a, total, lane);
-    unsigned j = pre;
     while (m) {
-        const int c = __ffs(m) - 1;
+        const uint32_t c = (uint32_t)__ffs(m) - 1u;
         m &= m - 1u;
-        const unsigned long long idx = j < sl.n0 ? sl.b0 + j : sl.b1 + (j - sl.n0);
-        if (idx < a.rec_cap) {
-            *reinterpret_cast<uint2 *>(a.rec + idx) = make_uint2(r.cell, (uint32_t)(col0 + c - r.seg0) << 16 | rank);
-        }
+        const unsigned long long idx = (j < sl.n0 ? sl.b0 : sl.b1) + j;
+        if (idx < cap)
+            *reinterpret_cast<uint2 *>(rec + idx) = make_uint2(cell, (off0 + c) << 16 | rank);
         ++rank;
         ++j;
     }
 }
 
-// One staged tile of nu units whose first (job-local) column is c0.  CHECK
-// adds the strict-upper-triangle test (col > row), row < n and col < n; it is
-// only needed on diagonal items, the last (partial) band and an odd last column.
-template <int L, bool CHECK>
-__device__ __forceinline__ void tile_pass(const PairArgs &a, const uint4 *tile, int nu, int32_t c0, const RowCtx &r,
-                                          uint32_t &rank, int lane)
-{
-    using U = Unit<L>;
-    for (int u = 0; u < nu; ++u) {
-        const uint4 *src = tile + u * U::kVec;
-        if constexpr (U::kTwo) {
-            uint32_t sel[16];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                if (v < U::kUsed) {
-                    const uint4 q = src[v];
-                    sel[4 * v] = q.x;
-                    sel[4 * v + 1] = q.y;
-                    sel[4 * v + 2] = q.z;
-                    sel[4 * v + 3] = q.w;
-                } else {
-                    sel[4 * v] = sel[4 * v + 1] = sel[4 * v + 2] = sel[4 * v + 3] = 0u;
-                }
-            }
-            bool h0, h1;
-            myers_two<L>(r.p01, r.p23, sel, a.one, a.two, r.lim, h0, h1);
-            const int32_t col = c0 + 2 * u;
-            uint32_t m = (h0 ? 1u : 0u) | (h1 ? 2u : 0u);
-            if (CHECK)
-                m &= upper_mask<2>(r, col);
-            if (__any_sync(kFull, m != 0u))
-                emit_mask<2>(a, m, r, col, rank, lane);
-        } else {
-            static_assert(U::kUsed == 2, "one-lane units are two uint4");
-            uint32_t sel[8];
-            const uint4 q0 = src[0];
-            const uint4 q1 = src[1];
-            sel[0] = q0.x; sel[1] = q0.y; sel[2] = q0.z; sel[3] = q0.w;
-            sel[4] = q1.x; sel[5] = q1.y; sel[6] = q1.z; sel[7] = q1.w;
-            const bool h0 = myers_one<L>(r.p01, r.p23, sel, a.one, a.two, a.hi, r.lim);
-            const int32_t col = c0 + u;
-            uint32_t m = h0 ? 1u : 0u;
-            if (CHECK)
-                m &= upper_mask<1>(r, col);
-            if (__any_sync(kFull, m != 0u))
-                emit_mask<1>(a, m, r, col, rank, lane);
-        }
+// A row's match words in one staged unit: the unit's table at the offsets of
+// the row's characters.
+template <int L>
+struct TileEq {
+    uint32_t at[L];  // byte offsets in the ring
+    __device__ __forceinline__ Words2 operator()(int i, int j) const
+    {
+        const uint2 v = *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(&g_tile[0][0]) + at[i] +
+                                                         j * slice::unit_pos_bytes());
+        return Words2{v.x, v.y};
     }
-}
+};
 
-// Byte lanes (editDist 5..8): one unit = 4 columns against the thread's row.
-template <int L, int MODE, bool CHECK>
-__device__ __forceinline__ void tile_pass_band(const PairArgs &a, const uint4 *tile, int nu, int32_t c0,
-                                               const RowCtx &r, const uint32_t (&W)[L], const BandConst &q,
-                                               uint32_t &rank, int lane)
-{
-    static_assert(MODE == kModeByte, "the nibble form runs in pair_kernel_nib");
-    using BU = BandUnit<MODE>;
-    for (int u = 0; u < nu; ++u) {
-        const uint4 *src = tile + u * BU::kVec;
-        uint32_t sel[8];
+template <int L_, int K>
+struct LevelForm {
+    static constexpr int L = L_;
+    uint32_t k0;
+    __device__ __forceinline__ explicit LevelForm(const JobDesc &J) : k0(J.k > 0 ? kFull : 0u) {}
+    __device__ __forceinline__ Words2 hits(const TileEq<L> &eq) const { return slice::levels<L, K>(eq, k0); }
+};
+
+template <int L_, int W>
+struct DeltaForm {
+    static constexpr int L = L_;
+    uint32_t nk[5];
+    __device__ __forceinline__ explicit DeltaForm(const JobDesc &J)
+    {
 #pragma unroll
-        for (int v = 0; v < 2; ++v) {
-            if (8 * v < L) {
-                const uint4 t4 = src[v];
-                sel[4 * v] = t4.x;
-                sel[4 * v + 1] = t4.y;
-                sel[4 * v + 2] = t4.z;
-                sel[4 * v + 3] = t4.w;
-            } else {
-                sel[4 * v] = sel[4 * v + 1] = sel[4 * v + 2] = sel[4 * v + 3] = 0u;
-            }
-        }
-        const uint32_t he = myers::band_byte<L>(W, sel, q);
-        if (__any_sync(kFull, he != 0u)) {
-            const int32_t base_col = c0 + u * BU::kCols;
-            // hit flag of column q at bit 8q+7
-            uint32_t m = hit_columns(he, a);
-            if (CHECK)
-                m &= upper_mask<BU::kCols>(r, base_col);
-            if (!CHECK || __any_sync(kFull, m != 0u))
-                emit_mask<BU::kCols>(a, m, r, base_col, rank, lane);
-        }
+        for (int b = 0; b < 5; ++b)
+            nk[b] = ((J.k >> b) & 1) ? 0u : kFull;
     }
-}
+    __device__ __forceinline__ Words2 hits(const TileEq<L> &eq) const
+    {
+        slice::Planes da, db;
+        slice::deltas<L, W>(eq, da, db);
+        return Words2{slice::at_most(da, nk), slice::at_most(db, nk)};
+    }
+};
 
-// Column-unit geometry of a lane form.
-template <int L, int MODE>
-struct Geo {
-    static constexpr int kCols = MODE == kModeFull ? Unit<L>::kCols : BandUnit<MODE>::kCols;
-    static constexpr int kVec = MODE == kModeFull ? Unit<L>::kVec : BandUnit<MODE>::kVec;
-    static constexpr int kTile = MODE == kModeFull ? kTileCols : BandUnit<MODE>::kTileCols;
-    static_assert(kTile / kCols * kVec <= kTileCols * 2, "a tile must fit one staging slot");
+// What a thread carries from item to item.
+struct LoopState {
+    WarpSlots ws;
+    uint32_t parity;  // bit b: phase parity of ring slot b; kSkipped
+    bool aborted;
 };
 
 // One (band, segment) item of job J: stream the segment's column tiles through
-// the two-slot ring and test them against the band's rows.
-template <int L, int MODE>
-__device__ __forceinline__ void run_item(const PairArgs &a, const JobDesc &J, int band, int seg,
-                                         uint4 (*tile)[kSlotVec], uint64_t *bar, uint32_t &parity, bool &aborted)
+// the two-slot ring and test them against the band's rows, one per thread.
+template <class Form>
+__device__ __noinline__ LoopState run_item(const JobDesc *job, int band, int seg, LoopState state)
 {
-    using G = Geo<L, MODE>;
+    const JobDesc &J = *job;
+    constexpr int L = Form::L;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
+    const int32_t n = J.n;
     const int32_t row0 = band * kBandRows;
-    RowCtx r;
-    r.row = row0 + tid;
-    r.ok = r.row < J.n;
-    r.n = J.n;
-    r.lim = J.lim;
-    r.seg0 = seg << J.seg_shift;
-    r.cell = (uint32_t)(J.count_off + (long long)seg * J.n + r.row);
-    const uint32_t rword = a.words[J.word_off + (r.ok ? r.row : 0)];
-    uint32_t W[MODE == kModeFull ? 1 : L];
-    BandConst q;
-    if constexpr (MODE == kModeFull) {
-        row_pools<L>(rword, r.p01, r.p23);
-    } else {
-        myers::band_windows<L, MODE>(rword, J.w, W);
-        q.vp0 = J.vp0;
-        q.bm = J.bm;
-        q.c = J.cmask;
-        q.k = J.kthr;
-        q.one = a.one;
-        q.h16 = a.hi;
+    const int32_t row = row0 + tid;
+    const int32_t seg0 = seg << J.seg_shift;
+    const uint32_t cell = (uint32_t)(J.count_off + (long long)seg * n + row);
+    uint32_t at[L];  // table offset of the row's character at each position
+    {
+        const uint32_t w = g_args.words[J.word_off + (row < n ? row : 0)];
+#pragma unroll
+        for (int i = 0; i < L; ++i)
+            at[i] = ((w >> (2 * i)) & 3u) * 8u;
     }
+    const Form form(J);
     // c_lo is a multiple of 256 (segments and bands are), so units never
     // straddle a segment
     const int32_t c_lo = (int32_t)max((long long)seg << J.seg_shift, (long long)row0);
-    const int32_t c_hi = (int32_t)min((long long)(seg + 1) << J.seg_shift, (long long)J.n);
+    const int32_t c_hi = (int32_t)min((long long)(seg + 1) << J.seg_shift, (long long)n);
     const long long row_end = (long long)row0 + kBandRows;
-    const bool check = ((long long)c_lo < row_end) || (row_end > (long long)J.n) ||
-                       (G::kCols > 1 && (c_hi % G::kCols) != 0);
-    const int ntiles = (c_hi - c_lo + G::kTile - 1) / G::kTile;
-    const uint4 *units = a.units + J.unit_off;
+    // col > row, row < n and col < n only need a look on diagonal items, the
+    // last (partial) band and a partial last unit
+    const bool check = ((long long)c_lo < row_end) || (row_end > (long long)n) || (c_hi % kUnitCols) != 0;
+    const int ntiles = (c_hi - c_lo + kTileCols - 1) / kTileCols;
+    const uint4 *units = g_args.units + J.unit_off;
     uint32_t rank = 0;
+    const uint32_t one = g_args.one;
+    const bool emit = g_args.emit != 0;
+    EdgeRecord *rec = g_args.rec;
+    const unsigned long long cap = g_args.rec_cap;
+    const long long wait_cycles = g_args.wait_cycles;
     // test hook: the first tile of the kernel's first item is never copied
-    if (a.skip_first_copy && J.item_off == 0 && band == 0 && seg == 0)
-        parity |= kSkipped;
+    if (g_args.skip_first_copy && J.item_off == 0 && band == 0 && seg == 0)
+        state.parity |= kSkipped;
 
     if (tid == 0) {
         for (int t = 0; t < 2 && t < ntiles; ++t)
-            if (!(t == 0 && (parity & kSkipped)))
-                ring_issue<G::kTile, G::kCols, G::kVec>(tile, bar, t, units, c_lo + t * G::kTile, c_hi);
+            if (!(t == 0 && (state.parity & kSkipped)))
+                ring_issue<L>(t, units, c_lo + t * kTileCols, c_hi);
     }
     for (int t = 0; t < ntiles; ++t) {
         const int b = t & 1;
         bool timed_out = false;
         const long long t_start = clock64();
-        while (!mbar_try_wait(&bar[b], (parity >> b) & 1u)) {
-            if (clock64() - t_start > a.wait_cycles) {
+        while (!mbar_try_wait(&g_bar[b], (state.parity >> b) & 1u)) {
+            if (clock64() - t_start > wait_cycles) {
                 timed_out = true;
                 break;
             }
         }
-        parity ^= 1u << b;
+        state.parity ^= 1u << b;
         // uniform decision: every thread leaves together if any gave up
         if (__syncthreads_or(timed_out)) {
             if (tid == 0)
-                ring_note_abort(a, b, !(t == 0 && (parity & kSkipped)), t + 1 < ntiles);
-            parity &= ~kSkipped;
-            aborted = true;
-            return;
+                ring_note_abort(b, !(t == 0 && (state.parity & kSkipped)), t + 1 < ntiles);
+            state.parity &= ~kSkipped;
+            state.aborted = true;
+            return state;
         }
-        parity &= ~kSkipped;
-        const int32_t c0 = c_lo + t * G::kTile;
-        const int nu = (min(G::kTile, c_hi - c0) + G::kCols - 1) / G::kCols;
-        if constexpr (MODE == kModeFull) {
-            if (check)
-                tile_pass<L, true>(a, tile[b], nu, c0, r, rank, lane);
-            else
-                tile_pass<L, false>(a, tile[b], nu, c0, r, rank, lane);
-        } else {
-            if (check)
-                tile_pass_band<L, MODE, true>(a, tile[b], nu, c0, r, W, q, rank, lane);
-            else
-                tile_pass_band<L, MODE, false>(a, tile[b], nu, c0, r, W, q, rank, lane);
+        state.parity &= ~kSkipped;
+        const int32_t c0 = c_lo + t * kTileCols;
+        const int nu = (min(kTileCols, c_hi - c0) + kUnitCols - 1) / kUnitCols;
+        const uint32_t at0 = (uint32_t)b * (kSlotVec * 16);
+        TileEq<L> eq;
+#pragma unroll 1
+        for (int u = 0; u < nu; ++u) {
+#pragma unroll
+            for (int i = 0; i < L; ++i)
+                eq.at[i] = imad(at[i], one, at0 + (uint32_t)u * (slice::unit_vec(L) * 16));
+            Words2 m = form.hits(eq);
+            const int32_t col0 = c0 + u * kUnitCols;
+            if (check) {
+                m.a &= upper_mask(row, n, col0);
+                m.b &= upper_mask(row, n, col0 + 32);
+            }
+            if (!__any_sync(kFull, (m.a | m.b) != 0u))
+                continue;
+            const uint32_t cnt = (uint32_t)(__popc(m.a) + __popc(m.b));
+            if (!emit) {
+                rank += cnt;
+                continue;
+            }
+            unsigned total, j;
+            warp_count_prefix(cnt, lane, total, j);
+            const Slots sl = take_slots(state.ws, total, lane);
+            write_hits(rec, cap, m.a, cell, (uint32_t)(col0 - seg0), rank, sl, j);
+            write_hits(rec, cap, m.b, cell, (uint32_t)(col0 - seg0) + 32u, rank, sl, j);
         }
         __syncthreads();
         if (tid == 0 && t + 2 < ntiles)
-            ring_issue<G::kTile, G::kCols, G::kVec>(tile, bar, b, units, c_lo + (t + 2) * G::kTile, c_hi);
+            ring_issue<L>(b, units, c_lo + (t + 2) * kTileCols, c_hi);
     }
-    if (r.ok)
-        a.counts[r.cell] = rank;
-    const unsigned hits = __reduce_add_sync(kFull, r.ok ? rank : 0u);
+    if (row < n)
+        g_args.counts[cell] = rank;
+    const unsigned hits = __reduce_add_sync(kFull, row < n ? rank : 0u);
     if (lane == 0 && hits != 0u)
-        atomicAdd(a.hit_count, (unsigned long long)hits);
-}
-
-template <int L>
-__device__ __forceinline__ void dispatch_mode(int mode, const PairArgs &a, const JobDesc &J, int band, int seg,
-                                              uint4 (*tile)[kSlotVec], uint64_t *bar, uint32_t &parity,
-                                              bool &aborted)
-{
-    if (mode == kModeByte)
-        run_item<L, kModeByte>(a, J, band, seg, tile, bar, parity, aborted);
-    else
-        run_item<L, kModeFull>(a, J, band, seg, tile, bar, parity, aborted);
-}
-
-template <int... Ls>
-__device__ __forceinline__ void dispatch_item(int L, const PairArgs &a, const JobDesc &J, int band, int seg,
-                                              uint4 (*tile)[kSlotVec], uint64_t *bar, uint32_t &parity,
-                                              bool &aborted, std::integer_sequence<int, Ls...>)
-{
-    ((L == Ls + 1 ? dispatch_mode<Ls + 1>(J.mode, a, J, band, seg, tile, bar, parity, aborted) : void()), ...);
+        atomicAdd(g_args.hit_count, (unsigned long long)hits);
+    return state;
 }
 
 // Local item -> (band, segment): bands are grouped by their first segment g;
@@ -659,291 +535,104 @@ __device__ __forceinline__ void decode_item(const JobDesc &J, long long li, int 
 }
 
 // The unused rest of each warp's record-slot chunk becomes sentinels.
-__device__ __forceinline__ void fill_slot_tails(const PairArgs &a)
+__device__ __forceinline__ void fill_slot_tails(const WarpSlots &w)
 {
-    const int tid = threadIdx.x;
-    const unsigned long long base = g_slot_base[tid >> 5];
-    const unsigned left = g_slot_left[tid >> 5];
-    for (unsigned k = tid & 31; k < left; k += 32) {
-        const unsigned long long idx = base + k;
-        if (idx < a.rec_cap)
-            *reinterpret_cast<uint2 *>(a.rec + idx) = make_uint2(kNoCell, 0u);
+    for (unsigned k = threadIdx.x & 31; k < w.left; k += 32) {
+        const unsigned long long idx = w.base + k;
+        if (idx < g_args.rec_cap)
+            *reinterpret_cast<uint2 *>(g_args.rec + idx) = make_uint2(kNoCell, 0u);
     }
 }
 
-// Persistent item loop of the nibble-lane kernel: the CTA takes (job, band,
-// segment) items of its job table from its work counter and runs them.
-template <typename RunItem>
-__device__ __forceinline__ void item_loop(const PairArgs &a, uint64_t *bar, long long &item_sh, RunItem &&run_one)
+// The item function of a job's (length, threshold class): level form K = 1
+// for every L, K = 2..4 for L > K, delta form W = 2..7 for L > 2 W.
+template <int K, int... Ls>
+__device__ __forceinline__ void dispatch_levels(const JobDesc *J, int band, int seg, LoopState &st,
+                                                std::integer_sequence<int, Ls...>)
+{
+    constexpr int kFirst = K == 1 ? 1 : K + 1;
+    ((J->L == Ls + kFirst ? (void)(st = run_item<LevelForm<Ls + kFirst, K>>(J, band, seg, st)) : void()), ...);
+}
+
+template <int W, int... Ls>
+__device__ __forceinline__ void dispatch_deltas(const JobDesc *J, int band, int seg, LoopState &st,
+                                                std::integer_sequence<int, Ls...>)
+{
+    constexpr int kFirst = 2 * W + 1;
+    ((J->L == Ls + kFirst ? (void)(st = run_item<DeltaForm<Ls + kFirst, W>>(J, band, seg, st)) : void()), ...);
+}
+
+// Persistent item loop: the CTA takes (job, band, segment) items of its job
+// table from its work counter and runs them.
+template <bool kLevels>
+__device__ __forceinline__ void pair_loop(const PairArgs &args)
 {
     const int tid = threadIdx.x;
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        g_args = args;
+        mbar_init(&g_bar[0], 1);
+        mbar_init(&g_bar[1], 1);
         mbar_fence_init();
     }
-    if ((tid & 31) == 0) {
-        g_slot_base[tid >> 5] = 0ull;
-        g_slot_left[tid >> 5] = 0u;
-    }
     __syncthreads();
-    uint32_t parity = 0u;  // bit b: phase parity of slot b
-    bool aborted = false;
+    LoopState st;
+    st.ws.base = 0ull;
+    st.ws.left = 0u;
+    st.parity = 0u;
+    st.aborted = false;
 
     for (;;) {
         if (tid == 0)
-            item_sh = (long long)atomicAdd(a.work, 1ull);
+            g_item = (long long)atomicAdd(args.work, 1ull);
         __syncthreads();
-        const long long item = item_sh;
-        if (item >= a.items || aborted)
+        const long long item = g_item;
+        if (item >= args.items)
             break;
-        const JobDesc J = a.jobs[find_job_by_item(a.jobs, a.njobs, item)];
+        const JobDesc *J = args.jobs + find_job_by_item(args.jobs, args.njobs, item);
         int band = 0, seg = 0;
-        decode_item(J, item - J.item_off, band, seg);
-        run_one(J, band, seg, parity, aborted);
-        if (aborted)
+        decode_item(*J, item - J->item_off, band, seg);
+#define IG_LEVELS(K)                                                                                      \
+    case K:                                                                                               \
+        dispatch_levels<K>(J, band, seg, st, std::make_integer_sequence<int, IG_MAX_LEN - (K > 1 ? K : 0)>{}); \
+        break;
+#define IG_DELTAS(W)                                                                                      \
+    case W:                                                                                               \
+        dispatch_deltas<W>(J, band, seg, st, std::make_integer_sequence<int, IG_MAX_LEN - 2 * W>{});      \
+        break;
+        if constexpr (kLevels) {
+            switch (J->cls) {
+                IG_LEVELS(1)
+                IG_LEVELS(2)
+                IG_LEVELS(3)
+                IG_LEVELS(4)
+            }
+        } else {
+            switch (J->cls) {
+                IG_DELTAS(2)
+                IG_DELTAS(3)
+                IG_DELTAS(4)
+                IG_DELTAS(5)
+                IG_DELTAS(6)
+                IG_DELTAS(7)
+            }
+        }
+#undef IG_LEVELS
+#undef IG_DELTAS
+        if (st.aborted)
             break;
         __syncthreads();
     }
-    if (aborted && tid == 0)
-        ring_drain(a, bar, parity);
-    if (a.emit && !aborted)
-        fill_slot_tails(a);
+    if (st.aborted && tid == 0)
+        ring_drain(st.parity);
+    if (args.emit && !st.aborted)
+        fill_slot_tails(st.ws);
 }
 
-// Full-Myers and byte-lane jobs: one row per thread, 256 threads per band.
-// (The item loop is written out here rather than shared with
-// pair_kernel_nib: through the shared template this kernel's register
-// allocation got a 256-byte stack frame and ran 9 % slower.)
-__global__ void __launch_bounds__(kBandRows, 6) pair_kernel(PairArgs a)
-{
-    __shared__ __align__(128) uint4 tile[2][kSlotVec];
-    __shared__ __align__(8) uint64_t bar[2];
-    __shared__ long long item_sh;
+// Level form (editDist <= 5).
+__global__ void __launch_bounds__(kBandRows, 3) pair_levels(PairArgs a) { pair_loop<true>(a); }
 
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_fence_init();
-    }
-    if ((tid & 31) == 0) {
-        g_slot_base[tid >> 5] = 0ull;
-        g_slot_left[tid >> 5] = 0u;
-    }
-    __syncthreads();
-    uint32_t parity = 0u;  // bit b: phase parity of slot b
-    bool aborted = false;
-
-    for (;;) {
-        if (tid == 0)
-            item_sh = (long long)atomicAdd(a.work, 1ull);
-        __syncthreads();
-        const long long item = item_sh;
-        if (item >= a.items || aborted)
-            break;
-        const JobDesc J = a.jobs[find_job_by_item(a.jobs, a.njobs, item)];
-        int band = 0, seg = 0;
-        decode_item(J, item - J.item_off, band, seg);
-        dispatch_item(J.L, a, J, band, seg, tile, bar, parity, aborted,
-                      std::make_integer_sequence<int, IG_MAX_LEN>{});
-        if (aborted)
-            break;
-        __syncthreads();
-    }
-    if (aborted && tid == 0)
-        ring_drain(a, bar, parity);
-    if (a.emit && !aborted)
-        fill_slot_tails(a);
-}
-
-// ---- nibble lanes (editDist <= 4): two rows per thread, 128 threads per band ----
-constexpr int kNibThreads = kBandRows / 2;
-
-// Records of one row's hits m (bit c: column col0 + c) at warp record numbers
-// j, j+1, ... of the slots sl.
-__device__ __forceinline__ void write_hits(const PairArgs &a, uint32_t m, const RowCtx &r, int32_t col0,
-                                           uint32_t &rank, const Slots &sl, unsigned &j)
-{
-    while (m) {
-        const int c = __ffs(m) - 1;
-        m &= m - 1u;
-        const unsigned long long idx = j < sl.n0 ? sl.b0 + j : sl.b1 + (j - sl.n0);
-        if (idx < a.rec_cap)
-            *reinterpret_cast<uint2 *>(a.rec + idx) = make_uint2(r.cell, (uint32_t)(col0 + c - r.seg0) << 16 | rank);
-        ++rank;
-        ++j;
-    }
-}
-
-// emit_mask for the two rows of a thread (at most 8 hits per unit).
-__device__ __forceinline__ void emit_two_rows(const PairArgs &a, uint32_t ma, uint32_t mb, const RowCtx &ra,
-                                              const RowCtx &rb, int32_t col0, uint32_t &rank_a, uint32_t &rank_b,
-                                              int lane)
-{
-    const uint32_t na = __popc(ma), nb = __popc(mb);
-    if (!a.emit) {
-        rank_a += na;
-        rank_b += nb;
-        return;
-    }
-    unsigned total, pre;
-    warp_count_prefix<4>(na + nb, lane, total, pre);
-    if (total == 0u)
-        return;
-    const Slots sl = take_slots(a, total, lane);
-    unsigned j = pre;
-    write_hits(a, ma, ra, col0, rank_a, sl, j);
-    write_hits(a, mb, rb, col0, rank_b, sl, j);
-}
-
-template <int L, bool CHECK>
-__device__ __forceinline__ void tile_pass_nib(const PairArgs &a, const uint4 *tile, int nu, int32_t c0,
-                                              const RowCtx &ra, const RowCtx &rb, const uint32_t (&W2)[L],
-                                              const BandConst &q, uint32_t &rank_a, uint32_t &rank_b, int lane)
-{
-    using BU = BandUnit<kModeNib>;
-    for (int u = 0; u < nu; ++u) {
-        const uint4 *src = tile + u * BU::kVec;
-        uint32_t sel[16];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            if (4 * v < L) {
-                const uint4 t4 = src[v];
-                sel[4 * v] = t4.x;
-                sel[4 * v + 1] = t4.y;
-                sel[4 * v + 2] = t4.z;
-                sel[4 * v + 3] = t4.w;
-            } else {
-                sel[4 * v] = sel[4 * v + 1] = sel[4 * v + 2] = sel[4 * v + 3] = 0u;
-            }
-        }
-        uint32_t he, ho;
-        myers::band_nib2<L>(W2, sel, q, he, ho);
-        if (__any_sync(kFull, (he | ho) != 0u)) {
-            const int32_t col0 = c0 + u * BU::kCols;
-            uint32_t ma = hit_columns(he, a), mb = hit_columns(ho, a);
-            if (CHECK) {
-                ma &= upper_mask<BU::kCols>(ra, col0);
-                mb &= upper_mask<BU::kCols>(rb, col0);
-            }
-            if (!CHECK || __any_sync(kFull, (ma | mb) != 0u))
-                emit_two_rows(a, ma, mb, ra, rb, col0, rank_a, rank_b, lane);
-        }
-    }
-}
-
-// One (band, segment) item of a nibble-lane job: thread t tests rows 2t and
-// 2t+1 of the band against the segment's columns, staged like run_item.
-template <int L>
-__device__ __forceinline__ void run_item_nib(const PairArgs &a, const JobDesc &J, int band, int seg,
-                                             uint4 (*tile)[kSlotVec], uint64_t *bar, uint32_t &parity,
-                                             bool &aborted)
-{
-    using BU = BandUnit<kModeNib>;
-    constexpr int kTile = BU::kTileCols;
-    static_assert(kTile / BU::kCols * BU::kVec <= kSlotVec, "a tile must fit one staging slot");
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int32_t row0 = band * kBandRows;
-    RowCtx ra, rb;
-    ra.row = row0 + 2 * tid;
-    rb.row = ra.row + 1;
-    ra.ok = ra.row < J.n;
-    rb.ok = rb.row < J.n;
-    ra.n = rb.n = J.n;
-    ra.lim = rb.lim = J.lim;
-    ra.seg0 = rb.seg0 = seg << J.seg_shift;
-    ra.cell = (uint32_t)(J.count_off + (long long)seg * J.n + ra.row);
-    rb.cell = ra.cell + 1u;
-    uint32_t W2[L];
-    {
-        uint32_t WB[L];
-        myers::band_windows<L, kModeNib>(a.words[J.word_off + (ra.ok ? ra.row : 0)], J.w, W2);
-        myers::band_windows<L, kModeNib>(a.words[J.word_off + (rb.ok ? rb.row : 0)], J.w, WB);
-#pragma unroll
-        for (int j = 0; j < L; ++j)
-            W2[j] |= WB[j] << 4;
-    }
-    BandConst q;
-    q.vp0 = J.vp0;
-    q.bm = J.bm;
-    q.c = J.cmask;
-    q.k = J.kthr;
-    q.one = a.one;
-    q.h16 = a.hi;
-    const int32_t c_lo = (int32_t)max((long long)seg << J.seg_shift, (long long)row0);
-    const int32_t c_hi = (int32_t)min((long long)(seg + 1) << J.seg_shift, (long long)J.n);
-    const long long row_end = (long long)row0 + kBandRows;
-    const bool check = ((long long)c_lo < row_end) || (row_end > (long long)J.n) || (c_hi % BU::kCols) != 0;
-    const int ntiles = (c_hi - c_lo + kTile - 1) / kTile;
-    const uint4 *units = a.units + J.unit_off;
-    uint32_t rank_a = 0, rank_b = 0;
-    // test hook: the first tile of the kernel's first item is never copied
-    if (a.skip_first_copy && J.item_off == 0 && band == 0 && seg == 0)
-        parity |= kSkipped;
-
-    if (tid == 0) {
-        for (int t = 0; t < 2 && t < ntiles; ++t)
-            if (!(t == 0 && (parity & kSkipped)))
-                ring_issue<kTile, BU::kCols, BU::kVec>(tile, bar, t, units, c_lo + t * kTile, c_hi);
-    }
-    for (int t = 0; t < ntiles; ++t) {
-        const int b = t & 1;
-        bool timed_out = false;
-        const long long t_start = clock64();
-        while (!mbar_try_wait(&bar[b], (parity >> b) & 1u)) {
-            if (clock64() - t_start > a.wait_cycles) {
-                timed_out = true;
-                break;
-            }
-        }
-        parity ^= 1u << b;
-        // uniform decision: every thread leaves together if any gave up
-        if (__syncthreads_or(timed_out)) {
-            if (tid == 0)
-                ring_note_abort(a, b, !(t == 0 && (parity & kSkipped)), t + 1 < ntiles);
-            parity &= ~kSkipped;
-            aborted = true;
-            return;
-        }
-        parity &= ~kSkipped;
-        const int32_t c0 = c_lo + t * kTile;
-        const int nu = (min(kTile, c_hi - c0) + BU::kCols - 1) / BU::kCols;
-        if (check)
-            tile_pass_nib<L, true>(a, tile[b], nu, c0, ra, rb, W2, q, rank_a, rank_b, lane);
-        else
-            tile_pass_nib<L, false>(a, tile[b], nu, c0, ra, rb, W2, q, rank_a, rank_b, lane);
-        __syncthreads();
-        if (tid == 0 && t + 2 < ntiles)
-            ring_issue<kTile, BU::kCols, BU::kVec>(tile, bar, b, units, c_lo + (t + 2) * kTile, c_hi);
-    }
-    if (ra.ok)
-        a.counts[ra.cell] = rank_a;
-    if (rb.ok)
-        a.counts[rb.cell] = rank_b;
-    const unsigned hits = __reduce_add_sync(kFull, (ra.ok ? rank_a : 0u) + (rb.ok ? rank_b : 0u));
-    if (lane == 0 && hits != 0u)
-        atomicAdd(a.hit_count, (unsigned long long)hits);
-}
-
-template <int... Ls>
-__device__ __forceinline__ void dispatch_nib(int L, const PairArgs &a, const JobDesc &J, int band, int seg,
-                                             uint4 (*tile)[kSlotVec], uint64_t *bar, uint32_t &parity,
-                                             bool &aborted, std::integer_sequence<int, Ls...>)
-{
-    ((L == Ls + 1 ? run_item_nib<Ls + 1>(a, J, band, seg, tile, bar, parity, aborted) : void()), ...);
-}
-
-__global__ void __launch_bounds__(kNibThreads, 12) pair_kernel_nib(PairArgs a)
-{
-    __shared__ __align__(128) uint4 tile[2][kSlotVec];
-    __shared__ __align__(8) uint64_t bar[2];
-    __shared__ long long item_sh;
-    item_loop(a, bar, item_sh, [&](const JobDesc J, int band, int seg, uint32_t &parity, bool &aborted) {
-        dispatch_nib(J.L, a, J, band, seg, tile, bar, parity, aborted, std::make_integer_sequence<int, IG_MAX_LEN>{});
-    });
-}
+// Delta form (editDist 6..16).
+__global__ void __launch_bounds__(kBandRows, 2) pair_deltas(PairArgs a) { pair_loop<false>(a); }
 
 // Per row: in-place exclusive prefix of its segment counts; degree -> out[row+1].
 // A row's cells (one per segment from its band's first segment on, a
@@ -1335,13 +1024,13 @@ int pair_grid(Ctx *ctx)
 {
     if (ctx->pair_grid == 0) {
         int bps = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, pair_kernel, kBandRows, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, pair_deltas, kBandRows, 0);
         cudaGetLastError();
         ctx->pair_grid = std::max(bps, 1) * ctx->sm_count;
         bps = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, pair_kernel_nib, kNibThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, pair_levels, kBandRows, 0);
         cudaGetLastError();
-        ctx->pair_grid_nib = std::max(bps, 1) * ctx->sm_count;
+        ctx->pair_grid_levels = std::max(bps, 1) * ctx->sm_count;
     }
     return ctx->pair_grid;
 }
@@ -1349,9 +1038,9 @@ int pair_grid(Ctx *ctx)
 // Device-side layout of a batch.
 struct BatchLayout {
     std::vector<JobDesc> desc;      // every job, in batch order
-    std::vector<JobDesc> desc_nib;  // nibble-lane jobs with items, item_off over their own items
-    std::vector<JobDesc> desc_gen;  // the other jobs with items (pair_kernel)
-    long long items_nib = 0, items_gen = 0;
+    std::vector<JobDesc> desc_levels;  // level-form jobs with items, item_off over their own items
+    std::vector<JobDesc> desc_deltas;  // the other jobs with items (pair_deltas)
+    long long items_levels = 0, items_deltas = 0;
     long long items = 0;
     long long units = 0;       // column units over all jobs
     long long pairs = 0;       // pair tests over the jobs with items (bounds the edges)
@@ -1363,25 +1052,26 @@ struct BatchLayout {
 // Each kernel (nibble lanes / the rest) gets items_per_cta[lane form] items
 // per CTA of its grid (the work split, 24 unless the autotuner chose
 // another), shared among its jobs in proportion to their pair tests.
-bool plan_batch(const std::vector<JobSpec> &jobs, int grid_gen, int grid_nib, const int (&items_per_cta)[3],
+bool plan_batch(const std::vector<JobSpec> &jobs, int grid_deltas, int grid_levels, const int (&items_per_cta)[3],
                 BatchLayout &out)
 {
     long double pairs_total[2] = {0, 0};
     for (const JobSpec &j : jobs)
-        pairs_total[myers::band_mode(j.len, j.min_ed) == kModeNib] += (long double)j.n * (j.n > 0 ? j.n - 1 : 0) / 2;
-    const long long grids[2] = {grid_gen, grid_nib};
+        pairs_total[slice::test_of(j.len, j.min_ed).levels] += (long double)j.n * (j.n > 0 ? j.n - 1 : 0) / 2;
+    const long long grids[2] = {grid_deltas, grid_levels};
     out = BatchLayout();
     for (const JobSpec &j : jobs) {
         JobDesc d{};
-        const int lane_form = myers::band_mode(j.len, j.min_ed);
-        const int kn = lane_form == kModeNib;
+        const slice::Test test = slice::test_of(j.len, j.min_ed);
+        const int kn = test.levels;
         const long double share = pairs_total[kn] > 0 ? ((long double)j.n * (j.n - 1) / 2) / pairs_total[kn] : 0;
-        const long long want = (long long)items_per_cta[lane_form] * grids[kn];
+        const long long want = (long long)items_per_cta[lane_form(j.len, j.min_ed)] * grids[kn];
         const PairPlan p = make_plan(j.n, std::max<long long>(1, (long long)(share * want)));
         d.word_off = j.word_off;
         d.n = j.n;
-        d.L = j.len;
-        d.lim = std::max(-64, std::min(64, j.min_ed - j.len));
+        d.L = test.L;
+        d.k = test.k;
+        d.cls = test.levels ? test.K : test.W;
         d.seg_shift = p.seg_shift;
         d.nseg = p.nseg;
         d.bands_per_seg = p.bands_per_seg;
@@ -1390,25 +1080,8 @@ bool plan_batch(const std::vector<JobSpec> &jobs, int grid_gen, int grid_nib, co
         d.unit_start = out.units;
         d.unit_off = out.unit_vec;
         d.count_off = out.counts;
-        d.mode = myers::band_mode(j.len, j.min_ed);
-        d.w = 0;
-        d.vp0 = d.bm = d.cmask = d.kthr = 0;
-        if (d.mode != kModeFull)
-            myers::band_constants(j.len, j.min_ed, d.mode, d.w, d.vp0, d.bm, d.cmask, d.kthr);
-        long long units, vec;
-        if (d.mode == kModeNib) {
-            units = ((long long)j.n + 3) / 4;
-            vec = 4;
-        } else if (d.mode == kModeByte) {
-            units = ((long long)j.n + 3) / 4;
-            vec = 2;
-        } else if (j.len <= 15) {
-            units = ((long long)j.n + 1) / 2;
-            vec = 4;
-        } else {
-            units = (long long)j.n;
-            vec = 2;
-        }
+        const long long units = ((long long)j.n + kUnitCols - 1) / kUnitCols;
+        const long long vec = slice::unit_vec(d.L);
         // n < 2 or min_ed <= 0: no pair can be an edge.  The job gets no items
         // and no segments, so its rows read no count cells (degree 0).
         const bool active = j.n >= 2 && j.min_ed >= 1;
@@ -1423,10 +1096,10 @@ bool plan_batch(const std::vector<JobSpec> &jobs, int grid_gen, int grid_nib, co
         out.desc.push_back(d);
         if (active && p.items > 0) {  // the kernel of its lane form takes its items
             JobDesc k = d;
-            long long &space = d.mode == kModeNib ? out.items_nib : out.items_gen;
+            long long &space = kn ? out.items_levels : out.items_deltas;
             k.item_off = space;
             space += p.items;
-            (d.mode == kModeNib ? out.desc_nib : out.desc_gen).push_back(k);
+            (kn ? out.desc_levels : out.desc_deltas).push_back(k);
         }
     }
     return out.counts < (1ll << 32);
@@ -1464,10 +1137,10 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     if (out && (s = ensure(ctx, ctx->scan_tmp, (size_t)((m + kScanChunk - 1) / kScanChunk) * sizeof(int64_t),
                            "scan workspace")) != IG_OK)
         return s;
-    // job buffer: all jobs | job-boundary offsets (compaction) | nibble-kernel jobs | pair_kernel jobs
+    // job buffer: all jobs | job-boundary offsets (compaction) | pair_levels jobs | pair_deltas jobs
     const size_t jbytes = B.desc.size() * sizeof(JobDesc);
     const size_t bbytes = (B.desc.size() + 1) * sizeof(int64_t);
-    const size_t nbytes = B.desc_nib.size() * sizeof(JobDesc), gbytes = B.desc_gen.size() * sizeof(JobDesc);
+    const size_t nbytes = B.desc_levels.size() * sizeof(JobDesc), gbytes = B.desc_deltas.size() * sizeof(JobDesc);
     const size_t table = jbytes + bbytes + nbytes + gbytes;
     if ((s = ensure(ctx, ctx->jobs, table, "job table")) != IG_OK)
         return s;
@@ -1479,9 +1152,9 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     std::memcpy(stage, B.desc.data(), jbytes);
     std::memset(stage + jbytes, 0, bbytes);
     if (nbytes)
-        std::memcpy(stage + jbytes + bbytes, B.desc_nib.data(), nbytes);
+        std::memcpy(stage + jbytes + bbytes, B.desc_levels.data(), nbytes);
     if (gbytes)
-        std::memcpy(stage + jbytes + bbytes + nbytes, B.desc_gen.data(), gbytes);
+        std::memcpy(stage + jbytes + bbytes + nbytes, B.desc_deltas.data(), gbytes);
     unsigned long long *host_flags = reinterpret_cast<unsigned long long *>(stage + flag_off);
     int64_t *host_bounds = reinterpret_cast<int64_t *>(stage + bound_off);
     char *jbase = static_cast<char *>(ctx->jobs.ptr);
@@ -1493,10 +1166,6 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     a.units = static_cast<const uint4 *>(ctx->sel.ptr);
     a.words = d_words;
     a.one = 1u;
-    a.two = 2u;
-    a.hi = 1u << 16;
-    a.gather = 0x00204081u;
-    a.h4 = 16u;
     a.work = flags + 0;
     a.rec_count = flags + 1;
     a.status = reinterpret_cast<int *>(flags + 2);
@@ -1507,8 +1176,8 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     a.emit = out ? 1 : 0;
     a.wait_cycles = ctx->wait_cycles;
     a.skip_first_copy = ctx->fault_tile_copy ? 1 : 0;
-    const int grid_nib = ctx->pair_grid_nib;
-    const unsigned prep_grid = (unsigned)((B.units + 255) / 256);
+    const int grid_levels = ctx->pair_grid_levels;
+    const unsigned prep_grid = (unsigned)((B.units + 7) / 8);  // one warp per unit
     const int n = out ? out->n : 0;
     // scatter grid: enough threads for the slots the pass can hand out
     const unsigned long long cap = rec_capacity(ctx);
@@ -1518,8 +1187,8 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         (uint64_t)(uintptr_t)stage,  table, (uint64_t)(uintptr_t)jbase, (uint64_t)(uintptr_t)d_words,
         (uint64_t)B.units,           (uint64_t)njobs, (uint64_t)(uintptr_t)ctx->sel.ptr,
         (uint64_t)(uintptr_t)flags,  (uint64_t)(uintptr_t)ctx->records.ptr, cap,
-        (uint64_t)(uintptr_t)ctx->counts.ptr, (uint64_t)a.emit, (uint64_t)B.items_gen, (uint64_t)B.items_nib,
-        B.desc_nib.size(),           B.desc_gen.size(), (uint64_t)grid, (uint64_t)grid_nib,
+        (uint64_t)(uintptr_t)ctx->counts.ptr, (uint64_t)a.emit, (uint64_t)B.items_deltas, (uint64_t)B.items_levels,
+        B.desc_levels.size(),           B.desc_deltas.size(), (uint64_t)grid, (uint64_t)grid_levels,
         out ? (uint64_t)(uintptr_t)out->row_ptr : 0, out ? (uint64_t)(uintptr_t)out->cols : 0, (uint64_t)n,
         (uint64_t)sgrid,             (uint64_t)(uintptr_t)ctx->scan_tmp.ptr, (uint64_t)B.counts,
         out ? (uint64_t)out->col_cap : 0, (uint64_t)a.wait_cycles, (uint64_t)a.skip_first_copy};
@@ -1542,21 +1211,21 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
             return e;
         phase_begin(ctx, IG_PHASE_PAIRS);
         PairArgs k = a;
-        if (B.items_gen > 0) {
+        if (B.items_deltas > 0) {
             k.jobs = reinterpret_cast<const JobDesc *>(jbase + jbytes + bbytes + nbytes);
-            k.njobs = (int)B.desc_gen.size();
-            k.items = B.items_gen;
-            pair_kernel<<<grid, kBandRows, 0, st>>>(k);
+            k.njobs = (int)B.desc_deltas.size();
+            k.items = B.items_deltas;
+            pair_deltas<<<grid, kBandRows, 0, st>>>(k);
             launched++;
             if ((e = cudaGetLastError()) != cudaSuccess)
                 return e;
         }
-        if (B.items_nib > 0) {
+        if (B.items_levels > 0) {
             k.jobs = reinterpret_cast<const JobDesc *>(jbase + jbytes + bbytes);
-            k.njobs = (int)B.desc_nib.size();
-            k.items = B.items_nib;
+            k.njobs = (int)B.desc_levels.size();
+            k.items = B.items_levels;
             k.work = flags + 4;
-            pair_kernel_nib<<<grid_nib, kNibThreads, 0, st>>>(k);
+            pair_levels<<<grid_levels, kBandRows, 0, st>>>(k);
             launched++;
             if ((e = cudaGetLastError()) != cudaSuccess)
                 return e;
@@ -1748,7 +1417,7 @@ ig_status count_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         return s;
     const int grid = pair_grid(ctx);
     BatchLayout B;
-    if (!plan_batch(jobs, grid, ctx->pair_grid_nib, ctx->items_per_cta, B))
+    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, B))
         return set_error(ctx, IG_ERR_CAPACITY, "batch too large for one launch");
     if (B.items == 0) {
         *edges = 0;
@@ -1775,9 +1444,9 @@ ig_status autotune(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec>
     static const int kCandidates[] = {6, 12, 24, 48, 96};
     if (jobs.empty())
         return set_error(ctx, IG_ERR_INPUT, "autotune needs a job");
-    const int mode = myers::band_mode(jobs[0].len, jobs[0].min_ed);
+    const int mode = lane_form(jobs[0].len, jobs[0].min_ed);
     for (const JobSpec &j : jobs)
-        if (myers::band_mode(j.len, j.min_ed) != mode)
+        if (lane_form(j.len, j.min_ed) != mode)
             return set_error(ctx, IG_ERR_INPUT, "autotune jobs must share one lane form");
     ig_status s = check_jobs(ctx, jobs);
     if (s != IG_OK)
@@ -1791,7 +1460,7 @@ ig_status autotune(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec>
         int tune[3] = {ctx->items_per_cta[0], ctx->items_per_cta[1], ctx->items_per_cta[2]};
         tune[mode] = c;
         BatchLayout B;
-        if (!plan_batch(jobs, grid, ctx->pair_grid_nib, tune, B))
+        if (!plan_batch(jobs, grid, ctx->pair_grid_levels, tune, B))
             return set_error(ctx, IG_ERR_CAPACITY, "batch too large for one launch");
         std::vector<int> sh;
         for (const JobDesc &d : B.desc)
@@ -1846,7 +1515,13 @@ ig_status autotune(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec>
     return s;
 }
 
-int lane_form(int len, int min_ed) { return myers::band_mode(len, min_ed); }
+// The classes of thresholds that the work split is kept for, as callers name
+// them (IG_LANES_*): editDist 1..4, 5..8 and the rest.
+int lane_form(int len, int min_ed)
+{
+    (void)len;
+    return min_ed >= 1 && min_ed <= 4 ? 1 : (min_ed >= 5 && min_ed <= 8 ? 2 : 0);
+}
 
 ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs)
 {
@@ -1862,7 +1537,7 @@ ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<Job
         long double pairs = 0;
         size_t largest = 0;
         for (const JobSpec &j : jobs)
-            if (j.n > 1 && j.min_ed > 0 && myers::band_mode(j.len, j.min_ed) == mode) {
+            if (j.n > 1 && j.min_ed > 0 && lane_form(j.len, j.min_ed) == mode) {
                 sub.push_back(j);
                 pairs += (long double)j.n * (j.n - 1) / 2;
                 if (j.n > sub[largest].n)
@@ -1895,7 +1570,7 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         return s;
     const int grid = pair_grid(ctx);
     BatchLayout B;
-    if (!plan_batch(jobs, grid, ctx->pair_grid_nib, ctx->items_per_cta, B))
+    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, B))
         return set_error(ctx, IG_ERR_CAPACITY, "batch too large for one launch");
     const int32_t n = (int32_t)B.rows;
     g->ctx = ctx;
@@ -1944,7 +1619,7 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
             return set_error(ctx, IG_ERR_STATE, "record slots exceeded a buffer sized for them twice");
         // slots of a rerun differ from this pass only by the chunk tails of
         // the warps (scheduling), so leave room for all of them
-        const size_t tails = ((size_t)grid * (kBandRows / 32) + (size_t)ctx->pair_grid_nib * (kNibThreads / 32)) *
+        const size_t tails = ((size_t)grid * (kBandRows / 32) + (size_t)ctx->pair_grid_levels * (kBandRows / 32)) *
                              kSlotChunk;
         const size_t want = (size_t)(total + total / 8) + tails + 1024;
         s = ensure(ctx, ctx->records, want * sizeof(EdgeRecord), "edge records");

@@ -35,9 +35,8 @@
 
 namespace ig {
 
-// Rows of one band = threads of one pair-test CTA; columns of one staged tile.
+// Rows of one band = threads of one pair-test CTA.
 constexpr int kBandRows = 256;
-constexpr int kTileCols = 256;
 
 // One emitted edge, 8 bytes: the index of its (row, segment) count cell, and
 // pos = (column offset within the segment) << 16 | rank of the column among
@@ -62,10 +61,9 @@ struct JobDesc {
     int64_t unit_start;  // first unit (prefix over jobs, in units)
     int64_t item_off;    // first (band, segment) work item (prefix over jobs)
     int64_t count_off;   // first per-(segment, row) count ([nseg][n] block)
-    int32_t n, L, lim;   // words, length, min_ed - L
+    int32_t n, L;        // words, length the pair test compares (slice::Test)
     int32_t seg_shift, nseg, bands_per_seg, nbands;
-    int32_t mode, w;     // lane form (full Myers / banded nibble / banded byte), band half-width
-    uint32_t vp0, bm, cmask, kthr;  // banded-mode constants
+    int32_t k, cls;      // hit iff distance <= k; level form: K, delta form: band half-width
 };
 
 // Host description of a job.
@@ -135,9 +133,9 @@ struct Ctx {
     int64_t launches = 0;
     // workspace
     DevBuf words, sel, counts, records, scan_tmp, flags, adj_tmp, jobs, aux, cols_ws;
-    int pair_grid = 0;                    // persistent CTAs of the pair kernel
-    int pair_grid_nib = 0;                // ... of the nibble-lane pair kernel
-    // work split per lane form (full Myers, nibble, byte lanes): target items
+    int pair_grid = 0;                    // persistent CTAs of the pair kernel, delta form
+    int pair_grid_levels = 0;             // ... of its level form
+    // work split per lane form (threshold class, IG_LANES_*): target items
     // per CTA, chosen by the autotuner (ig_ctx_autotune) or left at 24
     int items_per_cta[3] = {24, 24, 24};
     bool tuned[3] = {false, false, false};
@@ -237,8 +235,7 @@ PairPlan make_plan(int32_t n, long long target_items);
 // Device pipeline stages (ig_graph.cu).  Jobs index into d_words.
 ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, Graph *g);
 ig_status count_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, int64_t *edges);
-// Lane form of the pair kernel for (len, min_ed): kModeFull 0, kModeNib 1,
-// kModeByte 2 (ig_graph.cu).
+// Threshold class of (len, min_ed), IG_LANES_* (ig_graph.cu).
 int lane_form(int len, int min_ed);
 // Times the work-split candidates on `jobs` (one lane form) and keeps the
 // fastest for that lane form (ig_graph.cu).

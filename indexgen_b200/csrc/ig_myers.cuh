@@ -1,8 +1,8 @@
 // Device building blocks of the pair test, shared by the kernels that run it:
 // column-unit layout of the PRMT selector streams, the per-row match-mask
 // pools and the two Myers recurrences (two 16-bit lanes for L <= 15, one lane
-// for L = 16).  Used by the graph-building kernels and by the allocation-free
-// conflict count.
+// for L = 16).  Used by the nearest-centre assignment and by the
+// allocation-free conflict count.
 #pragma once
 
 #include <cstdint>
@@ -31,7 +31,6 @@ struct Unit {
     static constexpr int kVec = kTwo ? 4 : 2;       // uint4 per unit in the stream
     static constexpr int kUsed = kTwo ? (L + 3) / 4 : 2;  // uint4 read per unit
     static constexpr int kBytes = kVec * 16;
-    static constexpr int kTileUnits = kTileCols / kCols;
 };
 
 
@@ -173,167 +172,6 @@ __device__ __forceinline__ int myers_one_dist(uint32_t p01, uint32_t p23, const 
     myers_one_vectors<L>(p01, p23, sel, one, two, hi, pv, mv);
     constexpr uint32_t M = (L >= 32) ? 0xffffffffu : ((1u << L) - 1u);
     return L + __popc(pv & M) - __popc(mv & M);
-}
-
-// ---------------------------------------------------------------------------
-// Banded lanes.  For a threshold k = min_ed - 1 the decision ED <= k between
-// two equal-length strings only needs the diagonals |i - j| <= w, w = k/2
-// (Ukkonen): a path that leaves them costs more than k.  Each column's band is
-// a (2w+1)-bit vector, bit b <-> row i = j - w + b, and the recurrence is
-// Myers' with the band re-aligned by one row per column:
-//   D0 = (((Eq & VP) + VP) ^ VP) | Eq | VN          (carry out of the band dropped)
-//   HN = VP & D0;  HP = VN | ~(D0 | VP)
-//   Y  = D0 >> 1                                     (next column's alignment; 0 enters at the bottom)
-//   VN = Y & HP;   VP = HN | ~(Y | HP)
-// starting from VP = 1 on the band rows i >= 1 (rows <= 0 carry no delta) and
-// VN = 0.  The centre bit b = w is the main diagonal: D[L][L] = L - sum_j D0_j[w].
-// Many pair tests share one 32-bit word:
-//  * kNib  (w <= 1, min_ed <= 4): eight 4-bit lanes, band bits 0..2, bit 3 spare
-//    (two rows x four columns per thread)
-//  * kByte (w <= 3, min_ed <= 8): four 8-bit lanes, band bits 0..6, bit 7 spare
-// The spare bits of VP and Eq stay 0, so a lane's carry stops in its own spare
-// bit; D0 is masked to the band before it is shifted.  Y is not masked: its
-// spare bit may hold the next lane's bit 0, which reaches VN's spare bit only
-// (HP's spare bit is always 1, so VP's stays 0) and is masked out of D0.
-// Per character step kNib issues 11 ALU-pipe ops (1 PRMT, 8 LOP3, the add,
-// the shift) and one IMAD (the lane counter, off the critical path) for eight
-// pair tests (two rows x four columns), kByte the same for four (one row x
-// four columns).  (Moving the add and the shift to the FMA pipe as IMAD /
-// IMAD.HI, as an earlier form did, cut the ALU count to 9 but ran 7 % slower:
-// IMAD.HI is half rate and both sit on the recurrence's critical path.)  The
-// match masks of all lanes come from one PRMT on a window register W_j whose
-// byte c is the band window of Peq[c] at column j (kNib: two rows' windows,
-// one per nibble).  Lane counters of the centre bits (weight 2^w per byte)
-// are compared with the threshold by adding 128 - 2^w (L - k) per byte and
-// reading bit 7.
-// ---------------------------------------------------------------------------
-enum LaneMode : int { kModeFull = 0, kModeNib = 1, kModeByte = 2 };
-
-// Column units of the banded modes: 4 columns each.  kNib: one 32-bit word
-// per position (nibble l = char of column l in bits 0..15, bits 16..31 zero),
-// 16 words.  kByte: 16 bits per position (nibble l = char of column l), two
-// positions per word.
-template <int MODE>
-struct BandUnit {
-    static constexpr int kCols = 4;                          // columns per unit
-    static constexpr int kVec = MODE == kModeNib ? 4 : 2;    // uint4 per unit
-    static constexpr int kBytes = kVec * 16;
-    static constexpr int kTileCols = MODE == kModeNib ? 512 : 1024;  // columns per staged tile (8 KiB)
-};
-
-// Per-row band windows W_j, j = 0..L-1 (column j+1).
-template <int L, int MODE>
-__device__ __forceinline__ void band_windows(uint32_t word, int w, uint32_t (&W)[L])
-{
-    uint32_t pe[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-    for (int k = 0; k < L; ++k) {
-        const uint32_t c = (word >> (2 * k)) & 3u;
-        const uint32_t bit = 1u << k;
-        pe[0] |= (c == 0u) ? bit : 0u;
-        pe[1] |= (c == 1u) ? bit : 0u;
-        pe[2] |= (c == 2u) ? bit : 0u;
-        pe[3] |= (c == 3u) ? bit : 0u;
-    }
-    const uint32_t bandmask = (1u << (2 * w + 1)) - 1u;
-#pragma unroll
-    for (int j = 0; j < L; ++j) {
-        const int sh = j - w;  // rows i = j + 1 - w + b  <->  Peq bit i - 1
-        uint32_t x = 0;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            uint32_t v = sh >= 0 ? (pe[c] >> sh) : (pe[c] << (-sh));
-            x |= (v & bandmask) << (8 * c);
-        }
-        W[j] = x;
-    }
-}
-
-struct BandConst {
-    uint32_t vp0, bm, c, k;       // initial VP, band mask, centre mask, threshold constant
-    uint32_t one, h16;            // opaque 1 and 2^16 (IMAD / IMAD.HI operands)
-};
-
-// Eight pair tests: two rows A, B of one thread against four columns.  W2[j]
-// byte c holds row A's band window for character c in its low nibble and row
-// B's in its high nibble, so one PRMT with the column selector (nibble k =
-// character of column k at position j) yields all eight lanes: nibble 2k =
-// (A, column k), nibble 2k+1 = (B, column k).  Hit flags at bit 8k+7 of he
-// (row A) and ho (row B).
-template <int L>
-__device__ __forceinline__ void band_nib2(const uint32_t (&W2)[L], const uint32_t (&sel)[16], const BandConst &q,
-                                          uint32_t &he, uint32_t &ho)
-{
-    uint32_t vp = q.vp0, vn = 0u, acc = 0u, be = 0u, bo = 0u;
-#pragma unroll
-    for (int j = 0; j < L; ++j) {
-        const uint32_t eq = __byte_perm(W2[j], W2[j], sel[j]);
-        const uint32_t sum = (eq & vp) + vp;
-        const uint32_t d0 = ((sum ^ vp) | eq | vn) & q.bm;
-        const uint32_t hn = vp & d0;
-        const uint32_t hp = vn | ~(d0 | vp);
-        acc = imad(d0 & q.c, q.one, acc);  // off the critical path: on the FMA pipe
-        if ((j + 1) % 7 == 0 || j == L - 1) {  // nibble counters hold at most 7 steps of 2^w
-            be = imad(acc & 0x0f0f0f0fu, q.one, be);
-            bo = imad((acc >> 4) & 0x0f0f0f0fu, q.one, bo);
-            acc = 0u;
-        }
-        const uint32_t ys = d0 >> 1;  // spare bits may pick up a neighbour's bit 0
-        vn = ys & hp;
-        vp = hn | ~(ys | hp);
-    }
-    he = (be + q.k) & 0x80808080u;
-    ho = (bo + q.k) & 0x80808080u;
-}
-
-// Four pair tests (one row, four columns); hit flag of column l at bit 8l+7.
-template <int L>
-__device__ __forceinline__ uint32_t band_byte(const uint32_t (&W)[L], const uint32_t (&sel)[8], const BandConst &q)
-{
-    uint32_t vp = q.vp0, vn = 0u, acc = 0u;
-#pragma unroll
-    for (int j = 0; j < L; ++j) {
-        const uint32_t s = (j & 1) ? __umulhi(sel[j >> 1], q.h16) : sel[j >> 1];
-        const uint32_t eq = __byte_perm(W[j], W[j], s);
-        const uint32_t sum = (eq & vp) + vp;
-        const uint32_t d0 = ((sum ^ vp) | eq | vn) & q.bm;
-        const uint32_t hn = vp & d0;
-        const uint32_t hp = vn | ~(d0 | vp);
-        acc = imad(d0 & q.c, q.one, acc);  // off the critical path: on the FMA pipe
-        const uint32_t ys = d0 >> 1;
-        vn = ys & hp;
-        vp = hn | ~(ys | hp);
-    }
-    return imad(acc, q.one, q.k) & 0x80808080u;
-}
-
-// Per-job constants of the banded modes (host and device).
-__host__ __device__ inline int band_mode(int len, int min_ed)
-{
-    (void)len;
-    if (min_ed >= 1 && min_ed <= 4)
-        return kModeNib;
-    if (min_ed >= 5 && min_ed <= 8)
-        return kModeByte;
-    return kModeFull;
-}
-
-__host__ __device__ inline void band_constants(int len, int min_ed, int mode, int &w, uint32_t &vp0, uint32_t &bm,
-                                               uint32_t &c, uint32_t &k)
-{
-    const int kk = min_ed - 1;
-    w = kk / 2;
-    const int B = 2 * w + 1;
-    const uint32_t lane_bm = (1u << B) - 1u;
-    const uint32_t lane_vp = lane_bm & ~((1u << w) - 1u);  // band rows i >= 1: bits w..2w
-    const uint32_t rep = mode == kModeNib ? 0x11111111u : 0x01010101u;
-    bm = lane_bm * rep;
-    vp0 = lane_vp * rep;
-    c = (1u << w) * rep;
-    int thr = (1 << w) * (len - kk);
-    if (thr < 0)
-        thr = 0;
-    k = (uint32_t)(128 - thr) * 0x01010101u;
 }
 
 }  // namespace myers

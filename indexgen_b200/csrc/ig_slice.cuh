@@ -1,0 +1,284 @@
+// Bit-sliced pair test: one row against 32 columns per 32-bit word.
+//
+// Every word below holds one truth value for 32 columns, so an operation of
+// the distance recurrence is a three-input logic operation (LOP3) that serves
+// 32 pair tests.  What a thread needs of a column tile is, for row position i
+// and column position j, the word "which columns have the row's character x_i
+// at j": a lookup in a table of four one-hot words per column position, which
+// runs on the load/store pipe beside the logic.
+//
+// Two forms decide ED(x, y) <= k for words of one length L, both on the
+// diagonals |j - i| <= k/2 only: an alignment of equal-length words that
+// leaves them costs more than k (Ukkonen).
+//
+//  * levels (k <= 4): for every diagonal t and every e with |t| <= e <= k-|t|
+//    (less than |t| cannot be there, more cannot come back to the end) one
+//    word "the prefixes of lengths i and i+t are within e":
+//      S[t][e](i) = S[t][e](i-1) & Eq | S[t][e-1](i-1) | S[t+1][e-1](i-1)
+//                   | S[t-1][e-1](i)
+//    1 or 2 LOP3 each: 2, 6, 12, 20 per row position for k = 1..4, less what
+//    is constant at the start or never reaches S[0][k](L) at the end.
+//  * deltas (any k): Myers' horizontal and vertical differences, one bit pair
+//    per cell of the band:
+//      D0 = Eq | Mh | Mv;  Ph' = Mv | ~(D0 | Pv);  Mh' = Pv & D0
+//      Pv' = Mh | ~(D0 | Ph);  Mv' = Ph & D0
+//    5 LOP3 per cell (3 at the band's ends, where the difference to the cell
+//    outside is taken as +1: one more edit along the band's edge, never less
+//    than the true distance), and a carry-save sum of the main diagonal's
+//    steps, which is the distance.
+//
+// Counted with the constants of the start folded and what never reaches the
+// end left out, the levels take 113 LOP3 for 32 pair tests at L = 12, k = 3
+// (3.5 each), 258 at L = 16, k = 4 (8.1) and 80 at L = 15, k = 2 (2.5).  Bound
+// by the ALU pipe (64 lanes per clock and SM) except at k = 2, whose 43 table
+// words per 32 pair tests fill the shared-memory pipe (128 B per clock and SM)
+// first.  Measured on a B200 against the recurrence with one 4- or 8-bit lane
+// per pair test that this replaced (17.1, 43.3 and 21.3 operations per pair
+// test): builds of 201,601 words at L = 12, k = 3 21.56 -> 4.77 ms; 300,000 at
+// L = 16, k = 4 117.5 -> 21.8 ms; 150,001 at L = 15, k = 2 14.59 -> 2.08 ms;
+// 19,999 at L = 13, k = 6 (deltas) 0.95 -> 0.54 ms.
+#pragma once
+
+#include <cstdint>
+
+// host compilers warn about the pragma
+#ifdef __CUDA_ARCH__
+#define IG_UNROLL _Pragma("unroll")
+#else
+#define IG_UNROLL
+#endif
+
+namespace ig {
+namespace slice {
+
+constexpr int kMaxLevelK = 4;   // thresholds the level form is built for
+constexpr int kUnitCols = 64;   // columns per unit: two words, loaded together
+
+// 32 or 64 columns' truth values.
+struct Words2 {
+    uint32_t a, b;
+};
+
+// Unit of 64 columns as the kernels stage it: four one-hot pairs of words per
+// position, 32 L bytes.
+__host__ __device__ constexpr int unit_vec(int L) { return 2 * L; }  // uint4 per unit
+__host__ __device__ constexpr int unit_pos_bytes() { return 32; }
+
+// S[0][k](L) by levels.  eq(i, j): the columns whose character at j equals
+// the row's at i.  For k = 0 and 1 (K = 1) `k0` is 0 or all ones: hits at
+// distance 1 only count when it is set.
+template <int L, int K, class Eq>
+__host__ __device__ __forceinline__ Words2 levels(const Eq &eq, uint32_t k0)
+{
+    constexpr int W = K / 2;
+    Words2 S[2 * W + 1][K + 1];
+IG_UNROLL
+    for (int t = -W; t <= W; ++t)
+IG_UNROLL
+        for (int e = 0; e <= K; ++e) {
+            const uint32_t v = (t >= 0 && e >= t) ? 0xffffffffu : 0u;
+            S[t + W][e].a = S[t + W][e].b = v;
+        }
+IG_UNROLL
+    for (int i = 1; i <= L; ++i) {
+IG_UNROLL
+        for (int t = -W; t <= W; ++t) {
+            const int j = i + t;
+            const int at = t < 0 ? -t : t;
+            if (j < 0 || j > L)
+                continue;
+            if (j == 0) {  // the empty prefix: i = |t| edits
+IG_UNROLL
+                for (int e = 0; e <= K; ++e)
+                    S[t + W][e].a = S[t + W][e].b = e >= at ? 0xffffffffu : 0u;
+                continue;
+            }
+            const Words2 m = eq(i - 1, j - 1);
+IG_UNROLL
+            for (int e = K; e >= 0; --e) {
+                if (e < at || e > K - at)
+                    continue;
+                uint32_t va = S[t + W][e].a & m.a, vb = S[t + W][e].b & m.b;
+                if (e - 1 >= at) {
+                    va |= S[t + W][e - 1].a;
+                    vb |= S[t + W][e - 1].b;
+                }
+                if (t + 1 <= W && e - 1 >= (t + 1 < 0 ? -(t + 1) : t + 1) && e - 1 <= K - (t + 1 < 0 ? -(t + 1) : t + 1)) {
+                    va |= S[t + 1 + W][e - 1].a;
+                    vb |= S[t + 1 + W][e - 1].b;
+                }
+                if (t - 1 >= -W && j - 1 >= 0 && e - 1 >= (t - 1 < 0 ? 1 - t : t - 1) &&
+                    e - 1 <= K - (t - 1 < 0 ? 1 - t : t - 1)) {
+                    va |= S[t - 1 + W][e - 1].a;
+                    vb |= S[t - 1 + W][e - 1].b;
+                }
+                S[t + W][e].a = va;
+                S[t + W][e].b = vb;
+            }
+        }
+    }
+    Words2 r = S[W][K];
+    if (K == 1) {
+        r.a &= S[W][0].a | k0;
+        r.b &= S[W][0].b | k0;
+    }
+    return r;
+}
+
+// Carry-save sum of up to 16 one-bit words: plane[p] is bit p of the count.
+struct Planes {
+    uint32_t p[5];
+};
+
+// The distance in five bit planes, exact where it is at most 2W + 1 and
+// otherwise an upper bound greater than that (the band's own distance).
+template <int L, int W, class Eq>
+__host__ __device__ __forceinline__ void deltas(const Eq &eq, Planes &da, Planes &db)
+{
+    // horizontal differences of the row above, by diagonal (constant +1 at the top)
+    Words2 ph[2 * W + 1], mh[2 * W + 1];
+IG_UNROLL
+    for (int t = 0; t <= 2 * W; ++t) {
+        ph[t].a = ph[t].b = 0xffffffffu;
+        mh[t].a = mh[t].b = 0u;
+    }
+    // carry-save counter of the main diagonal's steps, two pending words a level
+    Words2 pend[5][2];
+    int have[5] = {0, 0, 0, 0, 0};
+IG_UNROLL
+    for (int i = 1; i <= L; ++i) {
+        Words2 pv, mv;  // vertical difference left of the cell
+        pv.a = pv.b = 0xffffffffu;
+        mv.a = mv.b = 0u;
+        Words2 nph[2 * W + 1], nmh[2 * W + 1];
+IG_UNROLL
+        for (int t = -W; t <= W; ++t) {
+            const int j = i + t;
+            nph[t + W].a = nph[t + W].b = 0xffffffffu;
+            nmh[t + W].a = nmh[t + W].b = 0u;
+            if (j < 1 || j > L)
+                continue;
+            const Words2 m = eq(i - 1, j - 1);
+            // the cell above lies on diagonal t + 1 of the row above; outside
+            // the band its difference is +1
+            uint32_t Pa = 0xffffffffu, Pb = 0xffffffffu, Ma = 0u, Mb = 0u;
+            if (t + 1 <= W) {
+                Pa = ph[t + 1 + W].a;
+                Pb = ph[t + 1 + W].b;
+                Ma = mh[t + 1 + W].a;
+                Mb = mh[t + 1 + W].b;
+            }
+            const uint32_t d0a = m.a | Ma | mv.a, d0b = m.b | Mb | mv.b;
+            nph[t + W].a = mv.a | ~(d0a | pv.a);
+            nph[t + W].b = mv.b | ~(d0b | pv.b);
+            nmh[t + W].a = pv.a & d0a;
+            nmh[t + W].b = pv.b & d0b;
+            pv.a = Ma | ~(d0a | Pa);
+            pv.b = Mb | ~(d0b | Pb);
+            mv.a = Pa & d0a;
+            mv.b = Pb & d0b;
+            if (t == 0) {
+                Words2 c;
+                c.a = ~d0a;
+                c.b = ~d0b;
+IG_UNROLL
+                for (int l = 0; l < 5; ++l) {
+                    if (have[l] < 2) {
+                        pend[l][have[l]] = c;
+                        ++have[l];
+                        break;
+                    }
+                    const Words2 x = pend[l][0], y = pend[l][1];
+                    Words2 s;
+                    s.a = x.a ^ y.a ^ c.a;
+                    s.b = x.b ^ y.b ^ c.b;
+                    Words2 k;
+                    k.a = (x.a & y.a) | (x.a & c.a) | (y.a & c.a);
+                    k.b = (x.b & y.b) | (x.b & c.b) | (y.b & c.b);
+                    pend[l][0] = s;
+                    have[l] = 1;
+                    c = k;
+                }
+            }
+        }
+IG_UNROLL
+        for (int t = 0; t <= 2 * W; ++t) {
+            ph[t] = nph[t];
+            mh[t] = nmh[t];
+        }
+    }
+    // settle the counter: half adders from the lowest level up
+IG_UNROLL
+    for (int l = 0; l < 5; ++l) {
+        if (have[l] == 2) {
+            const Words2 x = pend[l][0], y = pend[l][1];
+            Words2 c;
+            c.a = x.a & y.a;
+            c.b = x.b & y.b;
+            da.p[l] = x.a ^ y.a;
+            db.p[l] = x.b ^ y.b;
+            if (l + 1 < 5) {
+IG_UNROLL
+                for (int q = l + 1; q < 5; ++q) {
+                    if (have[q] < 2) {
+                        pend[q][have[q]] = c;
+                        ++have[q];
+                        break;
+                    }
+                    const Words2 u = pend[q][0], v = pend[q][1];
+                    Words2 s, k;
+                    s.a = u.a ^ v.a ^ c.a;
+                    s.b = u.b ^ v.b ^ c.b;
+                    k.a = (u.a & v.a) | (u.a & c.a) | (v.a & c.a);
+                    k.b = (u.b & v.b) | (u.b & c.b) | (v.b & c.b);
+                    pend[q][0] = s;
+                    have[q] = 1;
+                    c = k;
+                }
+            }
+        } else if (have[l] == 1) {
+            da.p[l] = pend[l][0].a;
+            db.p[l] = pend[l][0].b;
+        } else {
+            da.p[l] = db.p[l] = 0u;
+        }
+    }
+}
+
+// Columns whose count is at most k: nk[b] is 0 where bit b of k is set, else
+// all ones.
+__host__ __device__ __forceinline__ uint32_t at_most(const Planes &d, const uint32_t (&nk)[5])
+{
+    uint32_t gt = 0u;
+IG_UNROLL
+    for (int b = 0; b < 5; ++b)
+        gt = (d.p[b] & gt) | (d.p[b] & nk[b]) | (gt & nk[b]);
+    return ~gt;
+}
+
+// How a job's test runs: the length it is compared at, its threshold and its
+// form.  ED <= L always holds, so a threshold of L or more makes every pair a
+// hit: such a job runs as length 1 with threshold 1.
+struct Test {
+    int L, k;     // length and threshold of the form
+    int levels;   // 1 level form, 0 delta form
+    int K, W;     // level form: threshold class (1..4); delta form: half-width
+};
+
+__host__ __device__ inline Test test_of(int len, int min_ed)
+{
+    Test t;
+    t.L = len;
+    t.k = min_ed < 1 ? 0 : min_ed - 1;  // below 1 nothing is a hit and the job gets no items
+    if (t.k >= len) {
+        t.L = 1;
+        t.k = 1;
+    }
+    t.levels = t.k <= kMaxLevelK;
+    t.K = t.k < 1 ? 1 : t.k;
+    t.W = t.k / 2;
+    return t;
+}
+
+}  // namespace slice
+}  // namespace ig
