@@ -9,16 +9,20 @@
 // running minimum in registers; only the N int32 assignments leave the device.
 // Ties go to the lowest centre index, as np.argmin's first occurrence does.
 //
-// Layout: centres are the Myers patterns (their Peq pools are staged in
-// shared memory, 2048 per pass), words the texts: each thread holds the
-// selector stream of two words (two 16-bit lanes, L <= 15) or one (L = 16) in
-// registers and walks all centres with the full Myers recurrence of
-// ig_myers.cuh, reading the exact distance at the end.
+// Two kernels.  assign_sliced (9 centres or more): one word per thread against
+// 64 centres per step, bit-sliced (ig_slice.cuh), centre tables staged in
+// shared memory, 2,048 per pass.  assign_kernel (fewer, where most of a word's
+// bits would stand for no centre): centres are the Myers patterns (their Peq
+// pools in shared memory), words the texts: each thread holds the selector
+// stream of two words (two 16-bit lanes, L <= 15) or one (L = 16) in registers
+// and walks all centres with the full Myers recurrence of ig_myers.cuh,
+// reading the exact distance at the end.
 #include <algorithm>
 #include <climits>
 
 #include "ig_internal.h"
 #include "ig_myers.cuh"
+#include "ig_slice.cuh"
 
 namespace ig {
 namespace {
@@ -129,12 +133,208 @@ __global__ void __launch_bounds__(kAssignThreads) assign_kernel(const uint32_t *
         out[first + 1] = arg1;
 }
 
+// ---- bit-sliced over the centres ----
+//
+// The distances to 64 centres come out as bit planes (the delta form on a band
+// of half-width W), the nearest among them by one pass over the planes.  A
+// band distance of at most 2W + 1 is the true distance and a larger one means
+// a truly larger distance, so the nearest centre found is exact, ties
+// included, as soon as it is that near; a thread whose nearest is farther goes
+// over all centres again with the full matrix (full_nearest).  W is chosen so
+// that this happens to fewer than 1 thread in 1,000 on uniform words
+// (min_centres below).
+//
+// ALU-pipe bound: about 31 (W = 3) LOP3 per row position and 32 centres, 14.5
+// per distance at L = 14 with 64 centres, against 68.6 operations in
+// assign_kernel.  1,000,000 words on a B200, the whole call: L = 14, k = 64
+// 278.5 -> 76.5 us; L = 10 / 13 / 16, k = 64 214 / 263 / 638 -> 57 / 74 / 99 us,
+// k = 16 69 / 82 / 177 -> 41 / 52 / 68 us.
+constexpr int kUnitsPerPass = kCentreChunk / slice::kUnitCols;
+__shared__ __align__(16) uint4 g_centres[kUnitsPerPass * slice::unit_vec(IG_MAX_LEN)];  // 16 KiB
+
+template <int L, bool kHalf>
+struct CentreEq {
+    uint32_t at[L];  // byte offsets in the table
+    __device__ __forceinline__ slice::Words2 operator()(int i, int j) const
+    {
+        const char *p = reinterpret_cast<const char *>(g_centres) + at[i] + j * slice::unit_pos_bytes();
+        if constexpr (kHalf)
+            return slice::Words2{*reinterpret_cast<const uint32_t *>(p), 0u};
+        const uint2 v = *reinterpret_cast<const uint2 *>(p);
+        return slice::Words2{v.x, v.y};
+    }
+};
+
+// One word against a unit (or its first 32 centres) at byte offset `unit` of
+// the table; va / vb: its valid centres.
+template <int L, int W, bool kHalf>
+__device__ __forceinline__ void nearest_in_unit(const uint32_t (&at)[L], uint32_t one, uint32_t unit, uint32_t va,
+                                                uint32_t vb, int base, int &best, int &arg)
+{
+    CentreEq<L, kHalf> eq;
+#pragma unroll
+    for (int i = 0; i < L; ++i)
+        eq.at[i] = slice::imad(at[i], one, unit);
+    slice::Planes da, db;
+    slice::deltas<L, W>(eq, da, db);
+    int dist, col;
+    slice::smallest<L>(da, db, va, kHalf ? 0u : vb, dist, col);
+    if (dist < best) {
+        best = dist;
+        arg = base + col;
+    }
+}
+
+__device__ __forceinline__ uint32_t first_bits(int m) { return m >= 32 ? 0xffffffffu : (1u << m) - 1u; }
+
+// The staged pass's `cn` centres (global index of the first: c0).
+template <int L, int W>
+__device__ __forceinline__ void nearest_in_pass(const uint32_t (&at)[L], uint32_t one, int c0, int cn, int &best,
+                                                int &arg)
+{
+    constexpr uint32_t kBytes = slice::unit_vec(L) * 16;
+    int u = 0;
+#pragma unroll 1
+    for (; cn - u * slice::kUnitCols > 32; ++u)
+        nearest_in_unit<L, W, false>(at, one, (uint32_t)u * kBytes, 0xffffffffu,
+                                     first_bits(cn - u * slice::kUnitCols - 32), c0 + u * slice::kUnitCols, best, arg);
+    const int rest = cn - u * slice::kUnitCols;
+    if (rest > 0)
+        nearest_in_unit<L, W, true>(at, one, (uint32_t)u * kBytes, first_bits(rest), 0u, c0 + u * slice::kUnitCols,
+                                    best, arg);
+}
+
+// The same with the full matrix, 32 centres at a time (rare: kept out of the
+// main kernel's registers).
+template <int L>
+__device__ __noinline__ int2 full_nearest(uint32_t word, uint32_t one, int c0, int cn, int2 so_far)
+{
+    constexpr uint32_t kBytes = slice::unit_vec(L) * 16;
+    uint32_t at[L];
+#pragma unroll
+    for (int i = 0; i < L; ++i)
+        at[i] = ((word >> (2 * i)) & 3u) * 8u;
+#pragma unroll 1
+    for (int c = 0; c < cn; c += 32)
+        nearest_in_unit<L, L - 1, true>(at, one, (uint32_t)(c / slice::kUnitCols) * kBytes + (c & 32 ? 4u : 0u),
+                                        first_bits(cn - c), 0u, c0 + c, so_far.x, so_far.y);
+    return so_far;
+}
+
+// Stages the tables of centres [c0, c0 + cn).
+__device__ __forceinline__ void stage_centres(const uint32_t *__restrict__ centres, int c0, int cn, int L)
+{
+    const int lane = threadIdx.x & 31;
+    for (int u = threadIdx.x >> 5; u * slice::kUnitCols < cn; u += kAssignThreads / 32) {
+        const int a = u * slice::kUnitCols + lane, b = a + 32;
+        slice::write_unit(a < cn ? centres[c0 + a] : 0u, b < cn ? centres[c0 + b] : 0u, a < cn, b < cn, L, lane,
+                          reinterpret_cast<uint2 *>(g_centres + u * slice::unit_vec(L)));
+    }
+}
+
+template <int L, int W>
+__global__ void __launch_bounds__(kAssignThreads, 3) assign_sliced(const uint32_t *__restrict__ words, long long n,
+                                                                  const uint32_t *__restrict__ centres, int k,
+                                                                  int32_t *__restrict__ out, uint32_t one)
+{
+    const bool staged_once = k <= kCentreChunk;
+    if (staged_once) {
+        stage_centres(centres, 0, k, L);
+        __syncthreads();
+    }
+    for (long long first = blockIdx.x * (long long)kAssignThreads; first < n;
+         first += gridDim.x * (long long)kAssignThreads) {
+        const long long i = first + threadIdx.x;
+        const uint32_t word = i < n ? words[i] : 0u;
+        uint32_t at[L];
+#pragma unroll
+        for (int q = 0; q < L; ++q)
+            at[q] = ((word >> (2 * q)) & 3u) * 8u;
+        int best = INT_MAX, arg = 0;
+        for (int c0 = 0; c0 < k; c0 += kCentreChunk) {
+            const int cn = min(kCentreChunk, k - c0);
+            if (!staged_once) {
+                __syncthreads();  // the previous pass is done with the tables
+                stage_centres(centres, c0, cn, L);
+                __syncthreads();
+            }
+            nearest_in_pass<L, W>(at, one, c0, cn, best, arg);
+        }
+        if constexpr (2 * W + 1 < L) {
+            bool far = best > 2 * W + 1;
+            if (staged_once ? __any_sync(0xffffffffu, far) : __syncthreads_or(far)) {
+                int2 full = make_int2(INT_MAX, 0);
+                for (int c0 = 0; c0 < k; c0 += kCentreChunk) {
+                    const int cn = min(kCentreChunk, k - c0);
+                    if (!staged_once) {
+                        __syncthreads();
+                        stage_centres(centres, c0, cn, L);
+                        __syncthreads();
+                    }
+                    full = full_nearest<L>(word, one, c0, cn, full);
+                }
+                arg = full.y;
+            }
+        }
+        if (i < n)
+            out[i] = arg;
+    }
+}
+
+// Centres needed for a word's nearest to lie within 2W + 1 in all but 1 of
+// 1,000 cases (distances of 10^6 uniform word pairs per length): below that a
+// wider band is faster than the repeats.  W = 3 covers every distance up to
+// L = 7.
+//
+// A word costs the same for 1 to 32 centres, so below some count assign_kernel
+// wins: 1,000,000 words, k = 8 against k = 9, took 46 against 41 us at L = 10,
+// 53 against 54 at L = 13 and 101 against 69 at L = 16.
+constexpr int kSlicedMinCentres = 9;
+
+__host__ __device__ constexpr int min_centres(int L, int W)
+{
+    constexpr int w3[17] = {0, 1, 1, 1, 1, 1, 1, 1, 2, 3, 5, 8, 14, 24, 45, 89, 182};
+    constexpr int w4[17] = {0, 1, 1, 1, 1, 1, 1, 1, 1, 1, 2, 2, 3, 5, 7, 11, 17};
+    return W == 3 ? w3[L] : W == 4 ? w4[L] : 1;
+}
+
+template <int L, int W>
+void launch_sliced(Ctx *ctx, const uint32_t *words, long long n, const uint32_t *centres, int k, int32_t *out)
+{
+    const long long blocks = std::min<long long>((n + kAssignThreads - 1) / kAssignThreads, 3ll * ctx->sm_count);
+    assign_sliced<L, W><<<(unsigned)blocks, kAssignThreads, 0, ctx->stream>>>(words, n, centres, k, out, 1u);
+}
+
+// The narrowest band whose repeats are rare; lengths whose 9 centres always
+// suffice for W = 3 or 4 have no wider variant.
+template <int L>
+void launch_sliced_len(Ctx *ctx, const uint32_t *words, long long n, const uint32_t *centres, int k, int32_t *out)
+{
+    if (k >= min_centres(L, 3)) {
+        launch_sliced<L, 3>(ctx, words, n, centres, k, out);
+        return;
+    }
+    if constexpr (min_centres(L, 3) > kSlicedMinCentres) {
+        if (k >= min_centres(L, 4)) {
+            launch_sliced<L, 4>(ctx, words, n, centres, k, out);
+            return;
+        }
+        if constexpr (min_centres(L, 4) > kSlicedMinCentres)
+            launch_sliced<L, 5>(ctx, words, n, centres, k, out);
+    }
+}
+
 // The keyed minimum for the two-lane lengths (L <= 15) with at most 2^26
 // centres; the compare-and-select form otherwise.
 template <int L>
-void launch_assign_len(int grid, cudaStream_t st, const uint32_t *words, long long n, const uint32_t *centres, int k,
+void launch_assign_len(Ctx *ctx, int grid, const uint32_t *words, long long n, const uint32_t *centres, int k,
                        int32_t *out)
 {
+    const cudaStream_t st = ctx->stream;
+    if (k >= kSlicedMinCentres) {
+        launch_sliced_len<L>(ctx, words, n, centres, k, out);
+        return;
+    }
     constexpr uint32_t unit = 1u << kKeyShift;
     if constexpr (Unit<L>::kTwo) {
         if (k <= (int)kKeyIndexMask + 1) {
@@ -148,10 +348,10 @@ void launch_assign_len(int grid, cudaStream_t st, const uint32_t *words, long lo
 }
 
 template <int... Ls>
-void launch_assign(int L, int grid, cudaStream_t st, const uint32_t *words, long long n, const uint32_t *centres,
-                   int k, int32_t *out, std::integer_sequence<int, Ls...>)
+void launch_assign(Ctx *ctx, int L, int grid, const uint32_t *words, long long n, const uint32_t *centres, int k,
+                   int32_t *out, std::integer_sequence<int, Ls...>)
 {
-    ((L == Ls + 1 ? launch_assign_len<Ls + 1>(grid, st, words, n, centres, k, out) : void()), ...);
+    ((L == Ls + 1 ? launch_assign_len<Ls + 1>(ctx, grid, words, n, centres, k, out) : void()), ...);
 }
 
 __global__ void gather_words_kernel(const uint32_t *__restrict__ src, const int32_t *__restrict__ idx, long long n,
@@ -184,7 +384,7 @@ ig_status assign_centers(Ctx *ctx, const uint32_t *d_words, int64_t n, const uin
     const long long grid = (threads + kAssignThreads - 1) / kAssignThreads;
     if (grid > INT32_MAX)
         return set_error(ctx, IG_ERR_CAPACITY, "too many words for one assignment launch");
-    launch_assign(len, (int)grid, ctx->stream, d_words, n, d_centres, k, d_out,
+    launch_assign(ctx, len, (int)grid, d_words, n, d_centres, k, d_out,
                   std::make_integer_sequence<int, IG_MAX_LEN>{});
     ctx->launches++;
     const cudaError_t e = cudaGetLastError();

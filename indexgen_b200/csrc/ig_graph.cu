@@ -36,6 +36,7 @@ namespace ig {
 
 namespace {
 
+using slice::imad;
 using slice::kUnitCols;
 using slice::Words2;
 
@@ -131,10 +132,7 @@ __device__ __forceinline__ int find_job_by_row(const JobDesc *jobs, int njobs, l
 }
 
 // Column units of every job, one warp per unit of 64 columns: word (j, c, h)
-// has bit b set where column 32 h + b of the unit has character c at position
-// j.  A warp reads its 64 words, and each position's two character bits become
-// two ballots per 32 columns, from which lane 4 (j % 8) + c forms character
-// c's word.
+// has bit b set where column 32 h + b of the unit has character c at position j.
 __global__ void prep_units(const uint32_t *__restrict__ words, const JobDesc *__restrict__ jobs, int njobs,
                            long long total_units, uint4 *__restrict__ units)
 {
@@ -147,26 +145,8 @@ __global__ void prep_units(const uint32_t *__restrict__ words, const JobDesc *__
     const long long c0 = p * kUnitCols;
     const uint32_t *w = words + J.word_off;
     const bool oka = c0 + lane < J.n, okb = c0 + 32 + lane < J.n;
-    const uint32_t wa = oka ? w[c0 + lane] : 0u;
-    const uint32_t wb = okb ? w[c0 + 32 + lane] : 0u;
-    const uint32_t va = __ballot_sync(kFull, oka), vb = __ballot_sync(kFull, okb);
-    uint2 *out = reinterpret_cast<uint2 *>(units + J.unit_off + p * slice::unit_vec(J.L));
-    const uint32_t clo = (lane & 1) ? kFull : 0u, chi = (lane & 2) ? kFull : 0u;
-    for (int j0 = 0; j0 < J.L; j0 += 8) {
-        uint2 mine = make_uint2(0u, 0u);
-        for (int j = j0; j < min(j0 + 8, J.L); ++j) {
-            const uint32_t la = __ballot_sync(kFull, (wa >> (2 * j)) & 1u);
-            const uint32_t ha = __ballot_sync(kFull, (wa >> (2 * j + 1)) & 1u);
-            const uint32_t lb = __ballot_sync(kFull, (wb >> (2 * j)) & 1u);
-            const uint32_t hb = __ballot_sync(kFull, (wb >> (2 * j + 1)) & 1u);
-            if ((lane >> 2) == j - j0) {
-                mine.x = ~((la ^ clo) | (ha ^ chi)) & va;
-                mine.y = ~((lb ^ clo) | (hb ^ chi)) & vb;
-            }
-        }
-        if (j0 + (lane >> 2) < J.L)
-            out[4 * j0 + lane] = mine;
-    }
+    slice::write_unit(oka ? w[c0 + lane] : 0u, okb ? w[c0 + 32 + lane] : 0u, oka, okb, J.L, lane,
+                      reinterpret_cast<uint2 *>(units + J.unit_off + p * slice::unit_vec(J.L)));
 }
 
 struct PairArgs {
@@ -243,16 +223,6 @@ __device__ __forceinline__ Slots take_slots(WarpSlots &w, unsigned total, int la
     w.base = b1 + need;
     w.left = take - need;
     return s;
-}
-
-// Integer multiply-add with an operand the compiler cannot see as a constant,
-// so it stays an IMAD on the FMA pipe instead of an add on the ALU pipe (the
-// pipe the logic operations saturate).
-__device__ __forceinline__ uint32_t imad(uint32_t a, uint32_t b, uint32_t c)
-{
-    uint32_t d;
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
 }
 
 // Warp total of cnt and this lane's exclusive prefix.  When no lane has more

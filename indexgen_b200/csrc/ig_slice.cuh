@@ -64,6 +64,44 @@ struct Words2 {
 __host__ __device__ constexpr int unit_vec(int L) { return 2 * L; }  // uint4 per unit
 __host__ __device__ constexpr int unit_pos_bytes() { return 32; }
 
+#ifdef __CUDACC__
+// A warp writes the unit of the 64 words it holds (wa in columns 0..31, wb in
+// 32..63, one per lane; lanes out of range, oka / okb false, match nothing) to
+// out: each position's two character bits become two ballots per 32 columns,
+// from which lane 4 (j % 8) + c forms character c's words.
+__device__ __forceinline__ void write_unit(uint32_t wa, uint32_t wb, bool oka, bool okb, int L, int lane, uint2 *out)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t va = __ballot_sync(kAll, oka), vb = __ballot_sync(kAll, okb);
+    const uint32_t clo = (lane & 1) ? kAll : 0u, chi = (lane & 2) ? kAll : 0u;
+    for (int j0 = 0; j0 < L; j0 += 8) {
+        uint2 mine = make_uint2(0u, 0u);
+        for (int j = j0; j < min(j0 + 8, L); ++j) {
+            const uint32_t la = __ballot_sync(kAll, (wa >> (2 * j)) & 1u);
+            const uint32_t ha = __ballot_sync(kAll, (wa >> (2 * j + 1)) & 1u);
+            const uint32_t lb = __ballot_sync(kAll, (wb >> (2 * j)) & 1u);
+            const uint32_t hb = __ballot_sync(kAll, (wb >> (2 * j + 1)) & 1u);
+            if ((lane >> 2) == j - j0) {
+                mine.x = ~((la ^ clo) | (ha ^ chi)) & va;
+                mine.y = ~((lb ^ clo) | (hb ^ chi)) & vb;
+            }
+        }
+        if (j0 + (lane >> 2) < L)
+            out[4 * j0 + lane] = mine;
+    }
+}
+
+// Integer multiply-add with an operand the compiler cannot see as a constant,
+// so it stays an IMAD on the FMA pipe instead of an add on the ALU pipe (the
+// pipe the logic operations saturate).
+__device__ __forceinline__ uint32_t imad(uint32_t a, uint32_t b, uint32_t c)
+{
+    uint32_t d;
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+#endif
+
 // S[0][k](L) by levels.  eq(i, j): the columns whose character at j equals
 // the row's at i.  For k = 0 and 1 (K = 1) `k0` is 0 or all ones: hits at
 // distance 1 only count when it is set.
@@ -72,29 +110,29 @@ __host__ __device__ __forceinline__ Words2 levels(const Eq &eq, uint32_t k0)
 {
     constexpr int W = K / 2;
     Words2 S[2 * W + 1][K + 1];
-IG_UNROLL
+    IG_UNROLL
     for (int t = -W; t <= W; ++t)
-IG_UNROLL
+        IG_UNROLL
         for (int e = 0; e <= K; ++e) {
             const uint32_t v = (t >= 0 && e >= t) ? 0xffffffffu : 0u;
             S[t + W][e].a = S[t + W][e].b = v;
         }
-IG_UNROLL
+    IG_UNROLL
     for (int i = 1; i <= L; ++i) {
-IG_UNROLL
+        IG_UNROLL
         for (int t = -W; t <= W; ++t) {
             const int j = i + t;
             const int at = t < 0 ? -t : t;
             if (j < 0 || j > L)
                 continue;
             if (j == 0) {  // the empty prefix: i = |t| edits
-IG_UNROLL
+                IG_UNROLL
                 for (int e = 0; e <= K; ++e)
                     S[t + W][e].a = S[t + W][e].b = e >= at ? 0xffffffffu : 0u;
                 continue;
             }
             const Words2 m = eq(i - 1, j - 1);
-IG_UNROLL
+            IG_UNROLL
             for (int e = K; e >= 0; --e) {
                 if (e < at || e > K - at)
                     continue;
@@ -125,9 +163,67 @@ IG_UNROLL
     return r;
 }
 
-// Carry-save sum of up to 16 one-bit words: plane[p] is bit p of the count.
+// Counts of up to 16 one-bit words: p[b] is bit b of the count.
 struct Planes {
     uint32_t p[5];
+};
+
+// Carry-save counter.  Level l keeps one or two words of weight 2^l; a third
+// goes through a full adder, whose carry arrives at the next level.  Which of
+// these a word meets depends only on how many arrived before it, so with the
+// row loop unrolled it is all known at compile time.
+struct Counter {
+    Words2 one[5], two[5];
+    int arrived[5];
+
+    __host__ __device__ __forceinline__ Counter()
+    {
+        IG_UNROLL
+        for (int l = 0; l < 5; ++l)
+            arrived[l] = 0;
+    }
+
+    __host__ __device__ __forceinline__ void add(int level, Words2 c)
+    {
+        bool moving = true;
+        IG_UNROLL
+        for (int l = 0; l < 5; ++l) {
+            if (l >= level && moving) {
+                arrived[l] += 1;
+                if (arrived[l] == 1) {
+                    one[l] = c;
+                    moving = false;
+                } else if (arrived[l] % 2 == 0) {
+                    two[l] = c;
+                    moving = false;
+                } else {
+                    const Words2 x = one[l], y = two[l];
+                    one[l].a = x.a ^ y.a ^ c.a;
+                    one[l].b = x.b ^ y.b ^ c.b;
+                    c.a = (x.a & y.a) | (x.a & c.a) | (y.a & c.a);
+                    c.b = (x.b & y.b) | (x.b & c.b) | (y.b & c.b);
+                }
+            }
+        }
+    }
+
+    // The count, by half adders from the lowest level up.
+    __host__ __device__ __forceinline__ void settle(Planes &da, Planes &db)
+    {
+        IG_UNROLL
+        for (int l = 0; l < 5; ++l) {
+            if (arrived[l] == 0) {
+                da.p[l] = db.p[l] = 0u;
+            } else if (arrived[l] % 2 == 1) {
+                da.p[l] = one[l].a;
+                db.p[l] = one[l].b;
+            } else {
+                da.p[l] = one[l].a ^ two[l].a;
+                db.p[l] = one[l].b ^ two[l].b;
+                add(l + 1, Words2{one[l].a & two[l].a, one[l].b & two[l].b});
+            }
+        }
+    }
 };
 
 // The distance in five bit planes, exact where it is at most 2W + 1 and
@@ -137,21 +233,19 @@ __host__ __device__ __forceinline__ void deltas(const Eq &eq, Planes &da, Planes
 {
     // horizontal differences of the row above, by diagonal (constant +1 at the top)
     Words2 ph[2 * W + 1], mh[2 * W + 1];
-IG_UNROLL
+    IG_UNROLL
     for (int t = 0; t <= 2 * W; ++t) {
         ph[t].a = ph[t].b = 0xffffffffu;
         mh[t].a = mh[t].b = 0u;
     }
-    // carry-save counter of the main diagonal's steps, two pending words a level
-    Words2 pend[5][2];
-    int have[5] = {0, 0, 0, 0, 0};
-IG_UNROLL
+    Counter steps;  // of the main diagonal
+    IG_UNROLL
     for (int i = 1; i <= L; ++i) {
         Words2 pv, mv;  // vertical difference left of the cell
         pv.a = pv.b = 0xffffffffu;
         mv.a = mv.b = 0u;
         Words2 nph[2 * W + 1], nmh[2 * W + 1];
-IG_UNROLL
+        IG_UNROLL
         for (int t = -W; t <= W; ++t) {
             const int j = i + t;
             nph[t + W].a = nph[t + W].b = 0xffffffffu;
@@ -177,72 +271,38 @@ IG_UNROLL
             pv.b = Mb | ~(d0b | Pb);
             mv.a = Pa & d0a;
             mv.b = Pb & d0b;
-            if (t == 0) {
-                Words2 c;
-                c.a = ~d0a;
-                c.b = ~d0b;
-IG_UNROLL
-                for (int l = 0; l < 5; ++l) {
-                    if (have[l] < 2) {
-                        pend[l][have[l]] = c;
-                        ++have[l];
-                        break;
-                    }
-                    const Words2 x = pend[l][0], y = pend[l][1];
-                    Words2 s;
-                    s.a = x.a ^ y.a ^ c.a;
-                    s.b = x.b ^ y.b ^ c.b;
-                    Words2 k;
-                    k.a = (x.a & y.a) | (x.a & c.a) | (y.a & c.a);
-                    k.b = (x.b & y.b) | (x.b & c.b) | (y.b & c.b);
-                    pend[l][0] = s;
-                    have[l] = 1;
-                    c = k;
-                }
-            }
+            if (t == 0)
+                steps.add(0, Words2{~d0a, ~d0b});
         }
-IG_UNROLL
+        IG_UNROLL
         for (int t = 0; t <= 2 * W; ++t) {
             ph[t] = nph[t];
             mh[t] = nmh[t];
         }
     }
-    // settle the counter: half adders from the lowest level up
-IG_UNROLL
-    for (int l = 0; l < 5; ++l) {
-        if (have[l] == 2) {
-            const Words2 x = pend[l][0], y = pend[l][1];
-            Words2 c;
-            c.a = x.a & y.a;
-            c.b = x.b & y.b;
-            da.p[l] = x.a ^ y.a;
-            db.p[l] = x.b ^ y.b;
-            if (l + 1 < 5) {
-IG_UNROLL
-                for (int q = l + 1; q < 5; ++q) {
-                    if (have[q] < 2) {
-                        pend[q][have[q]] = c;
-                        ++have[q];
-                        break;
-                    }
-                    const Words2 u = pend[q][0], v = pend[q][1];
-                    Words2 s, k;
-                    s.a = u.a ^ v.a ^ c.a;
-                    s.b = u.b ^ v.b ^ c.b;
-                    k.a = (u.a & v.a) | (u.a & c.a) | (v.a & c.a);
-                    k.b = (u.b & v.b) | (u.b & c.b) | (v.b & c.b);
-                    pend[q][0] = s;
-                    have[q] = 1;
-                    c = k;
-                }
-            }
-        } else if (have[l] == 1) {
-            da.p[l] = pend[l][0].a;
-            db.p[l] = pend[l][0].b;
-        } else {
-            da.p[l] = db.p[l] = 0u;
-        }
+    steps.settle(da, db);
+}
+
+// The smallest distance among the columns ca | cb (at least one) and the first
+// column that has it, planes read from the highest down.
+template <int L>
+__host__ __device__ __forceinline__ void smallest(const Planes &da, const Planes &db, uint32_t ca, uint32_t cb,
+                                                  int &dist, int &col)
+{
+    dist = 0;
+    IG_UNROLL
+    for (int b = L < 16 ? 3 : 4; b >= 0; --b) {
+        const uint32_t za = ca & ~da.p[b], zb = cb & ~db.p[b];
+        const bool some = (za | zb) != 0u;
+        ca = some ? za : ca;
+        cb = some ? zb : cb;
+        dist |= some ? 0 : 1 << b;
     }
+#ifdef __CUDA_ARCH__
+    col = ca != 0u ? __ffs(ca) - 1 : __ffs(cb) + 31;
+#else
+    col = ca != 0u ? __builtin_ctz(ca) : 32 + __builtin_ctz(cb);
+#endif
 }
 
 // Columns whose count is at most k: nk[b] is 0 where bit b of k is set, else
@@ -250,7 +310,7 @@ IG_UNROLL
 __host__ __device__ __forceinline__ uint32_t at_most(const Planes &d, const uint32_t (&nk)[5])
 {
     uint32_t gt = 0u;
-IG_UNROLL
+    IG_UNROLL
     for (int b = 0; b < 5; ++b)
         gt = (d.p[b] & gt) | (d.p[b] & nk[b]) | (gt & nk[b]);
     return ~gt;
