@@ -22,6 +22,8 @@
 //   row_prefix      per-row exclusive prefix over its segments + degree
 //   scan            exclusive scan of degrees -> row_ptr (int64)
 //   scatter         cols[row_ptr[r] + prefix[cell] + rank] = col
+//   (dense jobs: the pair kernel stores every hit word instead of records, and
+//   expand_bits turns a cell's words into its columns at row_ptr + prefix)
 // The result is one upper CSR over the concatenated rows with global column
 // ids (block diagonal: jobs never share an edge), ascending per row and
 // bit-exact by construction (no sort, no dependence on scheduling).
@@ -161,6 +163,7 @@ struct PairArgs {
     unsigned long long *hit_count;  // pair tests that are edges (exact)
     EdgeRecord *rec;
     unsigned long long rec_cap;
+    uint2 *bits;  // hit words of the dense jobs
     uint32_t *counts;
     int *status;
     int emit;
@@ -312,6 +315,17 @@ __device__ __forceinline__ uint32_t upper_mask(int32_t row, int32_t n, int32_t c
     return row < n ? below_hi & ~below_lo : 0u;
 }
 
+// Hit words of a dense job: the words of 64-column unit u for rows 0.. up to
+// the end of the band whose diagonal the unit meets, unit after unit (the
+// triangle, in blocks of 256 x 256), so that a warp's 32 rows store 256
+// consecutive bytes.  Entry of (unit, row 0):
+__host__ __device__ __forceinline__ long long unit_bits(long long u)
+{
+    const long long c = u >> 2;
+    static_assert(kBandRows == 4 * slice::kUnitCols, "a band meets the diagonal in four units");
+    return 2 * kBandRows * c * (c + 1) + (u & 3) * kBandRows * (c + 1);
+}
+
 // Records of one word's hits m (bit c: column offset off0 + c in the segment)
 // at warp record numbers j, j+1, ... of the slots sl.  Ranks count the row's
 // hits in its (row, segment) cell in column order, so the scatter needs no
@@ -376,65 +390,93 @@ struct LoopState {
     bool aborted;
 };
 
+// What is the same for a whole item and only needed now and then: kept in
+// shared memory and read where it is used, not held in registers through the
+// pair loop (which is short of them).
+struct ItemShared {
+    const uint4 *units;
+    uint2 *bits;       // dense job: entry of (unit 0, first row of the band)
+    uint32_t cell;     // count cell of the band's first row
+    int32_t n, row0, seg0, c_lo, c_hi;
+};
+__shared__ ItemShared g_it;
+
+template <class T>
+__device__ __forceinline__ T now(const T &x)
+{
+    return *const_cast<const volatile T *>(&x);
+}
+
+// Ways out of the pair loop's common path (records of an item inside the
+// triangle): uniform bits.
+constexpr unsigned kCheck = 1u, kDense = 2u, kCountOnly = 4u;
+
 // One (band, segment) item of job J: stream the segment's column tiles through
 // the two-slot ring and test them against the band's rows, one per thread.
 template <class Form>
 __device__ __noinline__ LoopState run_item(const JobDesc *job, int band, int seg, LoopState state)
 {
-    const JobDesc &J = *job;
     constexpr int L = Form::L;
+    const JobDesc &J = *job;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    const int32_t n = J.n;
-    const int32_t row0 = band * kBandRows;
-    const int32_t row = row0 + tid;
-    const int32_t seg0 = seg << J.seg_shift;
-    const uint32_t cell = (uint32_t)(J.count_off + (long long)seg * n + row);
     uint32_t at[L];  // table offset of the row's character at each position
+    const Form form(J);
+    unsigned way = 0u;
+    int ntiles;
     {
-        const uint32_t w = g_args.words[J.word_off + (row < n ? row : 0)];
+        const int32_t n = J.n;
+        const int32_t row0 = band * kBandRows;
+        // c_lo is a multiple of 256 (segments and bands are), so units never
+        // straddle a segment
+        const int32_t c_lo = (int32_t)max((long long)seg << J.seg_shift, (long long)row0);
+        const int32_t c_hi = (int32_t)min((long long)(seg + 1) << J.seg_shift, (long long)n);
+        ntiles = (c_hi - c_lo + kTileCols - 1) / kTileCols;
+        // col > row, row < n and col < n only need a look on diagonal items,
+        // the last (partial) band and a partial last unit
+        const long long row_end = (long long)row0 + kBandRows;
+        if ((long long)c_lo < row_end || row_end > (long long)n || (c_hi % kUnitCols) != 0)
+            way |= kCheck;
+        if (!g_args.emit)
+            way |= kCountOnly;
+        else if (J.bit_off >= 0)
+            way |= kDense;
+        const uint32_t w = g_args.words[J.word_off + (row0 + tid < n ? row0 + tid : 0)];
 #pragma unroll
         for (int i = 0; i < L; ++i)
             at[i] = ((w >> (2 * i)) & 3u) * 8u;
+        // test hook: the first tile of the kernel's first item is never copied
+        if (g_args.skip_first_copy && J.item_off == 0 && band == 0 && seg == 0)
+            state.parity |= kSkipped;
+        if (tid == 0) {
+            g_it.units = g_args.units + J.unit_off;
+            g_it.bits = g_args.bits + J.bit_off + row0;
+            g_it.cell = (uint32_t)(J.count_off + (long long)seg * n + row0);
+            g_it.n = n;
+            g_it.row0 = row0;
+            g_it.seg0 = seg << J.seg_shift;
+            g_it.c_lo = c_lo;
+            g_it.c_hi = c_hi;
+            for (int t = 0; t < 2 && t < ntiles; ++t)
+                if (!(t == 0 && (state.parity & kSkipped)))
+                    ring_issue<L>(t, g_it.units, c_lo + t * kTileCols, c_hi);
+        }
     }
-    const Form form(J);
-    // c_lo is a multiple of 256 (segments and bands are), so units never
-    // straddle a segment
-    const int32_t c_lo = (int32_t)max((long long)seg << J.seg_shift, (long long)row0);
-    const int32_t c_hi = (int32_t)min((long long)(seg + 1) << J.seg_shift, (long long)n);
-    const long long row_end = (long long)row0 + kBandRows;
-    // col > row, row < n and col < n only need a look on diagonal items, the
-    // last (partial) band and a partial last unit
-    const bool check = ((long long)c_lo < row_end) || (row_end > (long long)n) || (c_hi % kUnitCols) != 0;
-    const int ntiles = (c_hi - c_lo + kTileCols - 1) / kTileCols;
-    const uint4 *units = g_args.units + J.unit_off;
-    uint32_t rank = 0;
     const uint32_t one = g_args.one;
-    const bool emit = g_args.emit != 0;
-    EdgeRecord *rec = g_args.rec;
-    const unsigned long long cap = g_args.rec_cap;
-    const long long wait_cycles = g_args.wait_cycles;
-    // test hook: the first tile of the kernel's first item is never copied
-    if (g_args.skip_first_copy && J.item_off == 0 && band == 0 && seg == 0)
-        state.parity |= kSkipped;
-
-    if (tid == 0) {
-        for (int t = 0; t < 2 && t < ntiles; ++t)
-            if (!(t == 0 && (state.parity & kSkipped)))
-                ring_issue<L>(t, units, c_lo + t * kTileCols, c_hi);
-    }
+    uint32_t rank = 0;
     for (int t = 0; t < ntiles; ++t) {
         const int b = t & 1;
         bool timed_out = false;
         const long long t_start = clock64();
         while (!mbar_try_wait(&g_bar[b], (state.parity >> b) & 1u)) {
-            if (clock64() - t_start > wait_cycles) {
+            if (clock64() - t_start > now(g_args.wait_cycles)) {
                 timed_out = true;
                 break;
             }
         }
         state.parity ^= 1u << b;
-        // uniform decision: every thread leaves together if any gave up
+        // uniform decision: every thread leaves together if any gave up (and
+        // the item's shared values are there for all)
         if (__syncthreads_or(timed_out)) {
             if (tid == 0)
                 ring_note_abort(b, !(t == 0 && (state.parity & kSkipped)), t + 1 < ntiles);
@@ -443,8 +485,8 @@ __device__ __noinline__ LoopState run_item(const JobDesc *job, int band, int seg
             return state;
         }
         state.parity &= ~kSkipped;
-        const int32_t c0 = c_lo + t * kTileCols;
-        const int nu = (min(kTileCols, c_hi - c0) + kUnitCols - 1) / kUnitCols;
+        const int32_t c0 = now(g_it.c_lo) + t * kTileCols;
+        const int nu = (min(kTileCols, now(g_it.c_hi) - c0) + kUnitCols - 1) / kUnitCols;
         const uint32_t at0 = (uint32_t)b * (kSlotVec * 16);
         TileEq<L> eq;
 #pragma unroll 1
@@ -454,30 +496,44 @@ __device__ __noinline__ LoopState run_item(const JobDesc *job, int band, int seg
                 eq.at[i] = imad(at[i], one, at0 + (uint32_t)u * (slice::unit_vec(L) * 16));
             Words2 m = form.hits(eq);
             const int32_t col0 = c0 + u * kUnitCols;
-            if (check) {
-                m.a &= upper_mask(row, n, col0);
-                m.b &= upper_mask(row, n, col0 + 32);
+            if (way & (kCheck | kDense)) {
+                const int32_t n = now(g_it.n), row = now(g_it.row0) + tid;
+                if (way & kCheck) {
+                    m.a &= upper_mask(row, n, col0);
+                    m.b &= upper_mask(row, n, col0 + 32);
+                }
+                if (way & kDense) {
+                    if (row < n)
+                        now(g_it.bits)[unit_bits(col0 / kUnitCols) + tid] = make_uint2(m.a, m.b);
+                    rank += (uint32_t)(__popc(m.a) + __popc(m.b));
+                    continue;
+                }
             }
             if (!__any_sync(kFull, (m.a | m.b) != 0u))
                 continue;
             const uint32_t cnt = (uint32_t)(__popc(m.a) + __popc(m.b));
-            if (!emit) {
+            if (way & kCountOnly) {
                 rank += cnt;
                 continue;
             }
             unsigned total, j;
             warp_count_prefix(cnt, lane, total, j);
             const Slots sl = take_slots(state.ws, total, lane);
-            write_hits(rec, cap, m.a, cell, (uint32_t)(col0 - seg0), rank, sl, j);
-            write_hits(rec, cap, m.b, cell, (uint32_t)(col0 - seg0) + 32u, rank, sl, j);
+            const uint32_t cell = now(g_it.cell) + (uint32_t)tid;
+            const uint32_t off = (uint32_t)(col0 - now(g_it.seg0));
+            EdgeRecord *rec = now(g_args.rec);
+            const unsigned long long cap = now(g_args.rec_cap);
+            write_hits(rec, cap, m.a, cell, off, rank, sl, j);
+            write_hits(rec, cap, m.b, cell, off + 32u, rank, sl, j);
         }
         __syncthreads();
         if (tid == 0 && t + 2 < ntiles)
-            ring_issue<L>(b, units, c_lo + (t + 2) * kTileCols, c_hi);
+            ring_issue<L>(b, now(g_it.units), c0 + 2 * kTileCols, now(g_it.c_hi));
     }
-    if (row < n)
-        g_args.counts[cell] = rank;
-    const unsigned hits = __reduce_add_sync(kFull, row < n ? rank : 0u);
+    const bool live = now(g_it.row0) + tid < now(g_it.n);
+    if (live)
+        g_args.counts[now(g_it.cell) + (uint32_t)tid] = rank;
+    const unsigned hits = __reduce_add_sync(kFull, live ? rank : 0u);
     if (lane == 0 && hits != 0u)
         atomicAdd(g_args.hit_count, (unsigned long long)hits);
     return state;
@@ -850,6 +906,99 @@ __global__ void scatter_records(const EdgeRecord *__restrict__ rec, const unsign
         scatter_one(__ldcs(r2 + i), jobs, njobs, ncells, row_ptr, counts, cols, col_cap);
 }
 
+// The columns of a dense job's (band, segment) item from its hit words, one
+// row per lane: every 256 columns a lane counts its hits, the warp lists them
+// row by row in shared memory (13 bits each: lane and column offset) and
+// copies the list out, so that a row's run of columns is written by
+// neighbouring lanes.  A list too long for the buffer (more than a quarter of
+// the pairs) is written by each lane on its own.
+//
+// Why words and not records: a record costs 16 bytes of traffic and some 45
+// instructions per hit (slot handling, a scattered 4-byte store), 17 ps a hit
+// on the 33 million of 40,000 words at L = 10, editDist 5; the words cost a
+// quarter of a byte per pair test and about 3 ps a hit.  The two meet near one
+// hit in 250 pair tests; dense_job takes the words from about one in 128.
+constexpr int kListMax = 2048;
+
+__global__ void __launch_bounds__(kBandRows) expand_bits(const uint2 *__restrict__ bits, const JobDesc *__restrict__ jobs,
+                                                         int njobs, const unsigned long long *__restrict__ hits,
+                                                         const int *__restrict__ status,
+                                                         const int64_t *__restrict__ row_ptr,
+                                                         const uint32_t *__restrict__ counts, int32_t *__restrict__ cols,
+                                                         unsigned long long col_cap)
+{
+    __shared__ uint16_t list[kBandRows / 32][kListMax];
+    __shared__ int64_t run[kBandRows / 32][32];  // where list entry 0 would go if it were lane l's
+    if (*hits > col_cap || *status != kStatusOk)
+        return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long item = blockIdx.x;
+    const JobDesc &J = jobs[find_job_by_item(jobs, njobs, item)];
+    int band = 0, seg = 0;
+    decode_item(J, item - J.item_off, band, seg);
+    const int32_t row = band * kBandRows + threadIdx.x;
+    const bool live = row < J.n;
+    const int blocks = (J.n + kBandRows - 1) / kBandRows;
+    const int per_seg = J.bands_per_seg;
+    int64_t at = 0;  // where the row's next column goes
+    if (live)
+        at = row_ptr[J.word_off + row] + (int64_t)counts[J.count_off + (long long)seg * J.n + row];
+    for (int cb = max(seg * per_seg, band); cb < min((seg + 1) * per_seg, blocks); ++cb) {
+        const int32_t col0 = cb * kBandRows;
+        uint2 w[4];
+        int cnt = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            w[q] = make_uint2(0u, 0u);
+            if (live && col0 + q * kUnitCols < J.n)
+                w[q] = __ldcs(bits + J.bit_off + unit_bits(4ll * cb + q) + row);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            cnt += __popc(w[q].x) + __popc(w[q].y);
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o)
+                incl += t;
+        }
+        const int total = __shfl_sync(kFull, incl, 31);
+        if (total == 0)
+            continue;
+        const int64_t base = J.word_off + col0;
+        if (total <= kListMax) {
+            int p = incl - cnt;
+            run[wid][lane] = at - p;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                uint32_t m = (q & 1) ? w[q >> 1].y : w[q >> 1].x;
+                while (m) {
+                    list[wid][p++] = (uint16_t)(lane << 8 | (q * 32 + __ffs(m) - 1));
+                    m &= m - 1u;
+                }
+            }
+            __syncwarp();
+            for (int e = lane; e < total; e += 32) {
+                const uint32_t v = list[wid][e];
+                cols[run[wid][v >> 8] + e] = (int32_t)(base + (v & 255u));
+            }
+            __syncwarp();
+        } else {
+            int64_t p = at;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                uint32_t m = (q & 1) ? w[q >> 1].y : w[q >> 1].x;
+                while (m) {
+                    cols[p++] = (int32_t)(base + q * 32 + __ffs(m) - 1);
+                    m &= m - 1u;
+                }
+            }
+        }
+        at += cnt;
+    }
+}
+
 ig_status ensure(Ctx *ctx, DevBuf &b, size_t bytes, const char *what)
 {
     if (b.bytes >= bytes && b.ptr)
@@ -1010,7 +1159,10 @@ struct BatchLayout {
     std::vector<JobDesc> desc;      // every job, in batch order
     std::vector<JobDesc> desc_levels;  // level-form jobs with items, item_off over their own items
     std::vector<JobDesc> desc_deltas;  // the other jobs with items (pair_deltas)
-    long long items_levels = 0, items_deltas = 0;
+    std::vector<JobDesc> desc_dense;  // dense jobs, item_off over their own items (expand_bits)
+    long long items_levels = 0, items_deltas = 0, items_dense = 0;
+    long long bits = 0;          // hit-word entries (8 bytes) of the dense jobs
+    long long record_pairs = 0;  // pair tests of the jobs that emit records
     long long items = 0;
     long long units = 0;       // column units over all jobs
     long long pairs = 0;       // pair tests over the jobs with items (bounds the edges)
@@ -1019,12 +1171,38 @@ struct BatchLayout {
     int64_t rows = 0;
 };
 
-// Each kernel (nibble lanes / the rest) gets items_per_cta[lane form] items
+// Jobs whose pair tests hit often enough for hit words (expand_bits): on
+// uniform words the share of pairs with distance < min_ed passes 1/128 between
+// min_ed = L/2 - 1 and L/2 for every length (10^6 sampled pairs each: 0.6 and
+// 4.2 % at L = 10, 0.2 and 1.7 % at L = 11, 0.7 and 3.7 % at L = 16).  Small
+// jobs are bound by launches, which a second kernel would add to.
+bool dense_job(const JobSpec &j) { return j.n >= 8192 && j.min_ed >= 1 && j.min_ed >= j.len / 2; }
+
+// Hit-word entries of a job of n words: the triangle of 256 x 256 blocks.
+long long job_bits(int32_t n)
+{
+    const long long blocks = ((long long)n + kBandRows - 1) / kBandRows;
+    return unit_bits(4 * blocks);
+}
+
+// Hit words take the record buffer's place: up to this much of it is allocated
+// for them (126,000 words), more only where the buffer has grown for records.
+constexpr size_t kBitsRoom = (size_t)1 << 30;
+
+// Each kernel (level form / delta form) gets items_per_cta[lane form] items
 // per CTA of its grid (the work split, 24 unless the autotuner chose
 // another), shared among its jobs in proportion to their pair tests.
+//
+// With `bits_limit` above 0, dense jobs (dense_job) keep hit words instead of
+// records as long as all of them fit that many bytes.
 bool plan_batch(const std::vector<JobSpec> &jobs, int grid_deltas, int grid_levels, const int (&items_per_cta)[3],
-                BatchLayout &out)
+                size_t bits_limit, BatchLayout &out)
 {
+    long double bits_total = 0;
+    for (const JobSpec &j : jobs)
+        if (dense_job(j))
+            bits_total += (long double)job_bits(j.n);
+    const bool use_bits = bits_total > 0 && bits_total * sizeof(uint2) <= (long double)bits_limit;
     long double pairs_total[2] = {0, 0};
     for (const JobSpec &j : jobs)
         pairs_total[slice::test_of(j.len, j.min_ed).levels] += (long double)j.n * (j.n > 0 ? j.n - 1 : 0) / 2;
@@ -1057,6 +1235,11 @@ bool plan_batch(const std::vector<JobSpec> &jobs, int grid_deltas, int grid_leve
         const bool active = j.n >= 2 && j.min_ed >= 1;
         if (!active)
             d.nseg = 0;
+        d.bit_off = -1;
+        if (active && use_bits && dense_job(j)) {
+            d.bit_off = out.bits;
+            out.bits += job_bits(j.n);
+        }
         out.items += active ? p.items : 0;
         out.pairs += active ? (long long)j.n * (j.n - 1) / 2 : 0;
         out.units += units;
@@ -1064,8 +1247,15 @@ bool plan_batch(const std::vector<JobSpec> &jobs, int grid_deltas, int grid_leve
         out.counts += (long long)d.nseg * j.n;
         out.rows = std::max<int64_t>(out.rows, j.word_off + j.n);
         out.desc.push_back(d);
-        if (active && p.items > 0) {  // the kernel of its lane form takes its items
+        if (active && p.items > 0) {  // the kernel of its form takes its items
             JobDesc k = d;
+            if (d.bit_off >= 0) {
+                k.item_off = out.items_dense;
+                out.items_dense += p.items;
+                out.desc_dense.push_back(k);
+            } else {
+                out.record_pairs += (long long)j.n * (j.n - 1) / 2;
+            }
             long long &space = kn ? out.items_levels : out.items_deltas;
             k.item_off = space;
             space += p.items;
@@ -1107,11 +1297,12 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     if (out && (s = ensure(ctx, ctx->scan_tmp, (size_t)((m + kScanChunk - 1) / kScanChunk) * sizeof(int64_t),
                            "scan workspace")) != IG_OK)
         return s;
-    // job buffer: all jobs | job-boundary offsets (compaction) | pair_levels jobs | pair_deltas jobs
+    // job buffer: all jobs | job-boundary offsets (compaction) | pair_levels jobs | pair_deltas jobs | dense jobs
     const size_t jbytes = B.desc.size() * sizeof(JobDesc);
     const size_t bbytes = (B.desc.size() + 1) * sizeof(int64_t);
     const size_t nbytes = B.desc_levels.size() * sizeof(JobDesc), gbytes = B.desc_deltas.size() * sizeof(JobDesc);
-    const size_t table = jbytes + bbytes + nbytes + gbytes;
+    const size_t dbytes = out ? B.desc_dense.size() * sizeof(JobDesc) : 0;
+    const size_t table = jbytes + bbytes + nbytes + gbytes + dbytes;
     if ((s = ensure(ctx, ctx->jobs, table, "job table")) != IG_OK)
         return s;
     // staging: the job table image | 4 flag words read back | job bounds read back
@@ -1125,6 +1316,8 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         std::memcpy(stage + jbytes + bbytes, B.desc_levels.data(), nbytes);
     if (gbytes)
         std::memcpy(stage + jbytes + bbytes + nbytes, B.desc_deltas.data(), gbytes);
+    if (dbytes)
+        std::memcpy(stage + jbytes + bbytes + nbytes + gbytes, B.desc_dense.data(), dbytes);
     unsigned long long *host_flags = reinterpret_cast<unsigned long long *>(stage + flag_off);
     int64_t *host_bounds = reinterpret_cast<int64_t *>(stage + bound_off);
     char *jbase = static_cast<char *>(ctx->jobs.ptr);
@@ -1140,8 +1333,11 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     a.rec_count = flags + 1;
     a.status = reinterpret_cast<int *>(flags + 2);
     a.hit_count = flags + 3;
-    a.rec = static_cast<EdgeRecord *>(ctx->records.ptr);
-    a.rec_cap = out ? rec_capacity(ctx) : 0;
+    // record buffer: hit words of the dense jobs | edge records
+    const size_t bits_bytes = out ? (size_t)B.bits * sizeof(uint2) : 0;
+    a.bits = static_cast<uint2 *>(ctx->records.ptr);
+    a.rec = reinterpret_cast<EdgeRecord *>(static_cast<char *>(ctx->records.ptr) + bits_bytes);
+    a.rec_cap = out ? rec_capacity(ctx) - bits_bytes / sizeof(EdgeRecord) : 0;
     a.counts = static_cast<uint32_t *>(ctx->counts.ptr);
     a.emit = out ? 1 : 0;
     a.wait_cycles = ctx->wait_cycles;
@@ -1150,9 +1346,10 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     const unsigned prep_grid = (unsigned)((B.units + 7) / 8);  // one warp per unit
     const int n = out ? out->n : 0;
     // scatter grid: enough threads for the slots the pass can hand out
-    const unsigned long long cap = rec_capacity(ctx);
-    const int sgrid = (int)std::min<unsigned long long>((std::min<unsigned long long>(cap, (unsigned long long)B.pairs) + 255) / 256 + 1,
-                                                        (unsigned long long)ctx->sm_count * 16);
+    const unsigned long long cap = a.rec_cap;
+    const int sgrid = (int)std::min<unsigned long long>(
+        (std::min<unsigned long long>(cap, (unsigned long long)B.record_pairs) + 255) / 256 + 1,
+        (unsigned long long)ctx->sm_count * 16);
     const std::vector<uint64_t> sig = {
         (uint64_t)(uintptr_t)stage,  table, (uint64_t)(uintptr_t)jbase, (uint64_t)(uintptr_t)d_words,
         (uint64_t)B.units,           (uint64_t)njobs, (uint64_t)(uintptr_t)ctx->sel.ptr,
@@ -1161,7 +1358,8 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         B.desc_levels.size(),           B.desc_deltas.size(), (uint64_t)grid, (uint64_t)grid_levels,
         out ? (uint64_t)(uintptr_t)out->row_ptr : 0, out ? (uint64_t)(uintptr_t)out->cols : 0, (uint64_t)n,
         (uint64_t)sgrid,             (uint64_t)(uintptr_t)ctx->scan_tmp.ptr, (uint64_t)B.counts,
-        out ? (uint64_t)out->col_cap : 0, (uint64_t)a.wait_cycles, (uint64_t)a.skip_first_copy};
+        out ? (uint64_t)out->col_cap : 0, (uint64_t)a.wait_cycles, (uint64_t)a.skip_first_copy,
+        (uint64_t)bits_bytes, (uint64_t)B.items_dense, dbytes, (uint64_t)(B.record_pairs > 0)};
     ctx->fault_tile_copy = false;  // the injected fault is one-shot
     int64_t launched = 0;
     s = run_graph(ctx, out ? 0 : 1, sig, out ? "build pass" : "count pass", [&]() -> cudaError_t {
@@ -1218,13 +1416,24 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
                 return cudaErrorLaunchFailure;
             phase_end(ctx, IG_PHASE_SCAN);
             phase_begin(ctx, IG_PHASE_SCATTER);
-            scatter_records<<<sgrid, 256, 0, st>>>(static_cast<const EdgeRecord *>(ctx->records.ptr), flags + 1,
-                                                    a.status, cap, d_jobs, njobs, (unsigned long long)B.counts,
-                                                    out->row_ptr, static_cast<const uint32_t *>(ctx->counts.ptr),
-                                                    out->cols, out->col_cap);
-            launched++;
-            if ((e = cudaGetLastError()) != cudaSuccess)
-                return e;
+            if (B.record_pairs > 0) {
+                scatter_records<<<sgrid, 256, 0, st>>>(a.rec, flags + 1, a.status, cap, d_jobs, njobs,
+                                                        (unsigned long long)B.counts, out->row_ptr,
+                                                        static_cast<const uint32_t *>(ctx->counts.ptr), out->cols,
+                                                        out->col_cap);
+                launched++;
+                if ((e = cudaGetLastError()) != cudaSuccess)
+                    return e;
+            }
+            if (B.items_dense > 0) {
+                expand_bits<<<(unsigned)B.items_dense, kBandRows, 0, st>>>(
+                    a.bits, reinterpret_cast<const JobDesc *>(jbase + jbytes + bbytes + nbytes + gbytes),
+                    (int)B.desc_dense.size(), a.hit_count, a.status, out->row_ptr,
+                    static_cast<const uint32_t *>(ctx->counts.ptr), out->cols, out->col_cap);
+                launched++;
+                if ((e = cudaGetLastError()) != cudaSuccess)
+                    return e;
+            }
             phase_end(ctx, IG_PHASE_SCATTER);
             phase_end(ctx, IG_PHASE_COMPACT);
             job_bounds<<<(unsigned)((njobs + 1 + 255) / 256), 256, 0, st>>>(out->row_ptr, d_jobs, njobs, n,
@@ -1306,6 +1515,7 @@ void trim_workspaces(Ctx *ctx, size_t keep_bytes)
         b->ptr = nullptr;
         b->bytes = 0;
     }
+    ctx->col_room = 0;
     cudaGetLastError();
 }
 
@@ -1387,7 +1597,7 @@ ig_status count_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         return s;
     const int grid = pair_grid(ctx);
     BatchLayout B;
-    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, B))
+    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, 0, B))
         return set_error(ctx, IG_ERR_CAPACITY, "batch too large for one launch");
     if (B.items == 0) {
         *edges = 0;
@@ -1430,7 +1640,7 @@ ig_status autotune(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec>
         int tune[3] = {ctx->items_per_cta[0], ctx->items_per_cta[1], ctx->items_per_cta[2]};
         tune[mode] = c;
         BatchLayout B;
-        if (!plan_batch(jobs, grid, ctx->pair_grid_levels, tune, B))
+        if (!plan_batch(jobs, grid, ctx->pair_grid_levels, tune, 0, B))
             return set_error(ctx, IG_ERR_CAPACITY, "batch too large for one launch");
         std::vector<int> sh;
         for (const JobDesc &d : B.desc)
@@ -1540,7 +1750,7 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         return s;
     const int grid = pair_grid(ctx);
     BatchLayout B;
-    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, B))
+    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, std::max(ctx->records.bytes, kBitsRoom), B))
         return set_error(ctx, IG_ERR_CAPACITY, "batch too large for one launch");
     const int32_t n = (int32_t)B.rows;
     g->ctx = ctx;
@@ -1560,18 +1770,22 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         g->edges = 0;
         return IG_OK;
     }
-    if (rec_capacity(ctx) == 0) {
-        s = ensure(ctx, ctx->records, (size_t)(1u << 22) * sizeof(EdgeRecord), "edge records");
+    const size_t bits_bytes = (size_t)B.bits * sizeof(uint2);
+    const size_t first_records = B.record_pairs > 0 ? (size_t)(1u << 22) * sizeof(EdgeRecord) : 0;
+    if (rec_capacity(ctx) == 0 || ctx->records.bytes < bits_bytes) {
+        s = ensure(ctx, ctx->records, bits_bytes + first_records, "edge records");
         if (s != IG_OK)
             return s;
     }
     unsigned long long slots = 0, total = 0;
     for (int attempt = 0;; ++attempt) {
         // columns go to a context workspace with room for every record slot
-        // the pass may fill (at most one per pair test), so the compaction
-        // runs in the same graph as the pair kernels, before the host has
-        // seen the edge count; the graph then gets an exact copy
-        const size_t col_cap = (size_t)std::min<unsigned long long>(rec_capacity(ctx), (unsigned long long)B.pairs);
+        // the pass may fill (at most one per pair test), or as many columns as
+        // a build on this context has needed, so the compaction runs in the
+        // same graph as the pair kernels, before the host has seen the edge
+        // count; the graph then gets an exact copy
+        const unsigned long long room = std::max(rec_capacity(ctx), ctx->col_room);
+        const size_t col_cap = (size_t)std::min<unsigned long long>(room, (unsigned long long)B.pairs);
         if ((s = ensure(ctx, ctx->cols_ws, std::max<size_t>(col_cap, 1) * sizeof(int32_t), "column workspace")) !=
             IG_OK)
             return s;
@@ -1583,18 +1797,21 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         s = run_pass(ctx, d_words, B, grid, &out, &slots, &total, g->job_edge_off.data());
         if (s != IG_OK)
             return s;
-        if (slots <= rec_capacity(ctx))
+        const unsigned long long record_cap = rec_capacity(ctx) - bits_bytes / sizeof(EdgeRecord);
+        if (slots <= record_cap && total <= out.col_cap)
             break;
         if (attempt > 0)
             return set_error(ctx, IG_ERR_STATE, "record slots exceeded a buffer sized for them twice");
-        // slots of a rerun differ from this pass only by the chunk tails of
-        // the warps (scheduling), so leave room for all of them
-        const size_t tails = ((size_t)grid * (kBandRows / 32) + (size_t)ctx->pair_grid_levels * (kBandRows / 32)) *
-                             kSlotChunk;
-        const size_t want = (size_t)(total + total / 8) + tails + 1024;
-        s = ensure(ctx, ctx->records, want * sizeof(EdgeRecord), "edge records");
-        if (s != IG_OK)
-            return s;
+        ctx->col_room = std::max(ctx->col_room, total + total / 8);
+        if (slots > record_cap) {
+            // slots of a rerun differ from this pass only by the chunk tails
+            // of the warps (scheduling), so leave room for all of them
+            const size_t tails = ((size_t)grid + (size_t)ctx->pair_grid_levels) * (kBandRows / 32) * kSlotChunk;
+            const size_t want = (size_t)(slots + slots / 8) + tails + 1024;
+            s = ensure(ctx, ctx->records, bits_bytes + want * sizeof(EdgeRecord), "edge records");
+            if (s != IG_OK)
+                return s;
+        }
     }
     g->edges = (int64_t)total;
     const int njobs = (int)B.desc.size();

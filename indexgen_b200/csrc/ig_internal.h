@@ -64,6 +64,7 @@ struct JobDesc {
     int32_t n, L;        // words, length the pair test compares (slice::Test)
     int32_t seg_shift, nseg, bands_per_seg, nbands;
     int32_t k, cls;      // hit iff distance <= k; level form: K, delta form: band half-width
+    int64_t bit_off;     // first entry of the job's hit words (dense jobs), else -1
 };
 
 // Host description of a job.
@@ -133,6 +134,7 @@ struct Ctx {
     int64_t launches = 0;
     // workspace
     DevBuf words, sel, counts, records, scan_tmp, flags, adj_tmp, jobs, aux, cols_ws;
+    unsigned long long col_room = 0;      // columns the largest build so far needed
     int pair_grid = 0;                    // persistent CTAs of the pair kernel, delta form
     int pair_grid_levels = 0;             // ... of its level form
     // work split per lane form (threshold class, IG_LANES_*): target items
@@ -187,7 +189,8 @@ struct Ctx {
     std::shared_ptr<HostBudget> host_budget = std::make_shared<HostBudget>(default_host_budget());
 };
 
-// Edge records that fit the context's record buffer.  Derived from the
+// Edge records that fit the context's record buffer (dense jobs keep their hit
+// words there instead).  Derived from the
 // buffer itself, so that a failed (re)allocation, which leaves the buffer
 // empty, can never leave a stale capacity behind.
 inline unsigned long long rec_capacity(const Ctx *ctx) { return ctx->records.bytes / sizeof(EdgeRecord); }
