@@ -62,10 +62,10 @@ ig_status ig_ctx_reserve(ig_ctx *ctx, int64_t edges);
 int64_t ig_ctx_launches(const ig_ctx *ctx);
 /* Per-phase device timing with CUDA events on the context's stream (off by
  * default).  Phases: IG_PHASE_PAIRS (the pair-test kernel), IG_PHASE_COMPACT
- * (row prefix + scan + scatter into CSR), IG_PHASE_PREP (selector streams),
- * and the three parts of IG_PHASE_COMPACT: IG_PHASE_PREFIX (per-row prefix
- * of the segment counts), IG_PHASE_SCAN (row offsets), IG_PHASE_SCATTER
- * (records into columns).  ig_ctx_phase_time returns the accumulated
+ * (row offsets + scatter into CSR), IG_PHASE_PREP (column units), and the
+ * parts of IG_PHASE_COMPACT: IG_PHASE_PREFIX (per-row prefix of the segment
+ * counts and, in the same kernel, the row offsets), IG_PHASE_SCAN (no longer
+ * apart: 0 launches), IG_PHASE_SCATTER (records or hit words into columns).  ig_ctx_phase_time returns the accumulated
  * milliseconds and launch count since profiling was last enabled. */
 #define IG_PHASE_PAIRS 0
 #define IG_PHASE_COMPACT 1

@@ -19,8 +19,8 @@
 //                   and emits hits as (cell, column offset, rank) records into
 //                   slots its warp takes in chunks, plus a per-(row, segment)
 //                   count.
-//   row_prefix      per-row exclusive prefix over its segments + degree
-//   scan            exclusive scan of degrees -> row_ptr (int64)
+//   row_offsets     per-row exclusive prefix over its segments + degree, and
+//                   the scan of the degrees -> row_ptr (int64)
 //   scatter         cols[row_ptr[r] + prefix[cell] + rank] = col
 //   (dense jobs: the pair kernel stores every hit word instead of records, and
 //   expand_bits turns a cell's words into its columns at row_ptr + prefix)
@@ -133,12 +133,30 @@ __device__ __forceinline__ int find_job_by_row(const JobDesc *jobs, int njobs, l
     return lo;
 }
 
+// What a pass starts from zero: its flag words, row_ptr[0] and the words of the
+// row-offset scan.  The first kernel clears them (a memset each costs a
+// graph node and its gap).
+constexpr int kFlagWords = 8;
+struct PassZero {
+    unsigned long long *flags;
+    int64_t *row_ptr;                // null: count-only pass
+    unsigned long long *scan_words;
+    long long scan_count;
+};
+
 // Column units of every job, one warp per unit of 64 columns: word (j, c, h)
 // has bit b set where column 32 h + b of the unit has character c at position j.
 __global__ void prep_units(const uint32_t *__restrict__ words, const JobDesc *__restrict__ jobs, int njobs,
-                           long long total_units, uint4 *__restrict__ units)
+                           long long total_units, uint4 *__restrict__ units, PassZero zero)
 {
-    const long long u = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (id < kFlagWords)
+        zero.flags[id] = 0ull;
+    if (zero.row_ptr && id == 0)
+        zero.row_ptr[0] = 0;
+    for (long long k = id; k < zero.scan_count; k += gridDim.x * (long long)blockDim.x)
+        zero.scan_words[k] = 0ull;
+    const long long u = id >> 5;
     const int lane = threadIdx.x & 31;
     if (u >= total_units)
         return;
@@ -681,7 +699,10 @@ __global__ void __launch_bounds__(kBandRows, 3) pair_levels(PairArgs a) { pair_l
 // Delta form (editDist 6..16).
 __global__ void __launch_bounds__(kBandRows, 2) pair_deltas(PairArgs a) { pair_loop<false>(a); }
 
-// Per row: in-place exclusive prefix of its segment counts; degree -> out[row+1].
+// Per row: in-place exclusive prefix of its segment counts, and the row
+// offsets row_ptr of all rows, in one launch (a row's degree, a scan of the
+// degrees over the blocks by decoupled look-back).
+//
 // A row's cells (one per segment from its band's first segment on, a
 // [segment][row] array) are split into kPrefixParts consecutive chunks, each
 // taken by its own thread: the threads of a warp hold 32 consecutive rows of
@@ -693,21 +714,79 @@ __global__ void __launch_bounds__(kBandRows, 2) pair_deltas(PairArgs a) { pair_l
 // (8 and 16 threads per row measured slower on the headline job: 0.048 and
 // 0.084 ms against 0.038 ms, the shorter chunks leaving each thread less to
 // overlap.)
+//
+// One launch where there were five (prefix, three of a scan, job bounds): with
+// the memsets and read-backs also folded into the first and last kernels a
+// build went from 13 graph nodes to 5, and 2,000 words at L = 12, editDist 4
+// from 122 to 100 us, 19,999 at L = 13, editDist 7 from 378 to 346.
+//
+// Look-back: a block takes its number from a ticket, so every block before it
+// is already running; it publishes its own degree sum, then adds up the
+// blocks before it from their published words, 32 at a time, until one holds
+// a complete prefix, and publishes its own.  A word is the sum in 62 bits
+// under two bits saying what it is (0 nothing, 1 the block's own sum, 2 the
+// prefix up to and including the block).  The wait is bounded like the pair
+// kernels' and ends in the same status.
 constexpr int kPrefixParts = 4;
 constexpr int kPrefixRows = 256 / kPrefixParts;
+constexpr unsigned long long kOwnSum = 1ull << 62, kPrefixSum = 2ull << 62, kSumMask = (1ull << 62) - 1;
 
-__global__ void __launch_bounds__(256) row_prefix(uint32_t *__restrict__ counts, const JobDesc *__restrict__ jobs,
-                                                  int njobs, int64_t rows, int64_t *__restrict__ out)
+// Sum of the degrees of all blocks before block b; lane-parallel in one warp.
+// False when the wait ran out.
+__device__ __forceinline__ bool look_back(const unsigned long long *words, int64_t b, long long wait_cycles,
+                                          int *status, unsigned long long &before)
+{
+    const int lane = threadIdx.x & 31;
+    before = 0ull;
+    const long long t0 = clock64();
+    for (int64_t end = b; end > 0; end -= 32) {
+        const int64_t i = end - 1 - lane;
+        unsigned long long w = kPrefixSum;  // before block 0: an empty prefix
+        for (;;) {
+            if (i >= 0)
+                w = *reinterpret_cast<const volatile unsigned long long *>(words + i);
+            if (__all_sync(kFull, w != 0ull))
+                break;
+            // every lane sees lane 0's view of the clock and of the status
+            const bool stop = clock64() - t0 > wait_cycles ||
+                              *reinterpret_cast<const volatile int *>(status) != kStatusOk;
+            if (__shfl_sync(kFull, (int)stop, 0))
+                return false;
+        }
+        const unsigned full = __ballot_sync(kFull, (w & kPrefixSum) != 0ull);
+        // lanes up to the nearest complete prefix count
+        const int last = full != 0u ? __ffs(full) - 1 : 31;
+        unsigned long long v = lane <= last ? (w & kSumMask) : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            v += __shfl_xor_sync(kFull, v, o);
+        before += v;
+        if (full != 0u)
+            break;
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(256) row_offsets(uint32_t *__restrict__ counts, const JobDesc *__restrict__ jobs,
+                                                   int njobs, int64_t rows, int64_t *__restrict__ out,
+                                                   unsigned long long *__restrict__ words, int *status,
+                                                   long long wait_cycles)
 {
     __shared__ uint32_t part_sum[kPrefixParts][kPrefixRows];
+    __shared__ unsigned long long half_sum, before_sh;
+    __shared__ int64_t block_sh;
+    if (threadIdx.x == 0)
+        block_sh = (int64_t)atomicAdd(words, 1ull);  // the ticket; block b's word is words[1 + b]
+    __syncthreads();
+    const int64_t block = block_sh;
     const int r = threadIdx.x % kPrefixRows, q = threadIdx.x / kPrefixRows;
-    const int64_t gr = blockIdx.x * (int64_t)kPrefixRows + r;
+    const int64_t gr = block * kPrefixRows + r;
     const bool live = gr < rows;
     uint32_t *p = nullptr;
     int64_t stride = 0;
     int len = 0;
     if (live) {
-        const JobDesc J = jobs[find_job_by_row(jobs, njobs, gr)];
+        const JobDesc &J = jobs[find_job_by_row(jobs, njobs, gr)];
         const int64_t row = gr - J.word_off;
         const int g = (int)(((row / kBandRows) * kBandRows) >> J.seg_shift);
         const int m = max(J.nseg - g, 0);
@@ -734,6 +813,39 @@ __global__ void __launch_bounds__(256) row_prefix(uint32_t *__restrict__ counts,
     }
     part_sum[q][r] = sum;
     __syncthreads();
+    // warps 0 and 1: the block's rows' degrees and their inclusive sums
+    unsigned long long incl = 0ull;
+    if (threadIdx.x < kPrefixRows) {
+        static_assert(kPrefixRows == 64, "two warps hold the block's rows");
+#pragma unroll
+        for (int t = 0; t < kPrefixParts; ++t)
+            incl += part_sum[t][r];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(kFull, incl, o);
+            if ((threadIdx.x & 31) >= o)
+                incl += t;
+        }
+        if (threadIdx.x == 31)
+            half_sum = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32 && threadIdx.x < kPrefixRows)
+        incl += half_sum;
+    if (threadIdx.x == kPrefixRows - 1)
+        *reinterpret_cast<volatile unsigned long long *>(words + 1 + block) = (block == 0 ? kPrefixSum : kOwnSum) | incl;
+    if (threadIdx.x >= 32 && threadIdx.x < 64) {  // the warp that holds the block's sum
+        unsigned long long before = 0ull;
+        const bool ok = look_back(words + 1, block, wait_cycles, status, before);
+        if (threadIdx.x == kPrefixRows - 1) {
+            if (!ok)
+                atomicCAS(status, kStatusOk, kStatusTimeout);
+            else if (block > 0)
+                *reinterpret_cast<volatile unsigned long long *>(words + 1 + block) = kPrefixSum | (before + incl);
+            before_sh = before;
+        }
+    }
+    // meanwhile the cells
     uint32_t acc = 0;
     for (int t = 0; t < q; ++t)
         acc += part_sum[t][r];
@@ -756,19 +868,28 @@ __global__ void __launch_bounds__(256) row_prefix(uint32_t *__restrict__ counts,
             acc += c;
         }
     }
-    if (live && q == kPrefixParts - 1)
-        out[gr + 1] = (int64_t)acc;
+    __syncthreads();
+    if (threadIdx.x < kPrefixRows && live)
+        out[gr + 1] = (int64_t)(before_sh + incl);
 }
 
-// Row offsets at job boundaries: out[j] = row_ptr[word_off_j], out[k] = row_ptr[rows].
-__global__ void job_bounds(const int64_t *__restrict__ row_ptr, const JobDesc *__restrict__ jobs, int njobs,
-                           int64_t rows, int64_t *__restrict__ out)
+// What a pass reports to the host, written by one block of its last kernel
+// straight into page-locked host memory: the four flag words, and row_ptr at
+// the job boundaries (out[j] = row_ptr[word_off_j], out[k] = row_ptr[rows]).
+struct Report {
+    const unsigned long long *flags;
+    unsigned long long *host_flags;
+    int64_t *host_bounds;
+    int64_t rows;
+};
+
+__device__ __forceinline__ void report(const Report &to, const int64_t *__restrict__ row_ptr,
+                                       const JobDesc *__restrict__ jobs, int njobs)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < njobs)
-        out[j] = row_ptr[jobs[j].word_off];
-    else if (j == njobs)
-        out[j] = row_ptr[rows];
+    for (int j = threadIdx.x; j <= njobs; j += blockDim.x)
+        to.host_bounds[j] = row_ptr[j < njobs ? jobs[j].word_off : to.rows];
+    if (threadIdx.x < 4)
+        to.host_flags[threadIdx.x] = to.flags[threadIdx.x];
 }
 
 // ---- inclusive scan of int64 in place: block scan, scan of block sums, add ----
@@ -906,8 +1027,10 @@ __global__ void scatter_records(const EdgeRecord *__restrict__ rec, const unsign
                                 const int *__restrict__ status, unsigned long long cap, const JobDesc *__restrict__ jobs,
                                 int njobs, unsigned long long ncells, const int64_t *__restrict__ row_ptr,
                                 const uint32_t *__restrict__ counts, int32_t *__restrict__ cols,
-                                unsigned long long col_cap)
+                                unsigned long long col_cap, Report to)
 {
+    if (blockIdx.x == 0)
+        report(to, row_ptr, jobs, njobs);
     const unsigned long long nrec = *d_slots;
     if (nrec > cap || *status != kStatusOk)
         return;
@@ -946,10 +1069,13 @@ __global__ void __launch_bounds__(kBandRows) expand_bits(const uint2 *__restrict
                                                          const int *__restrict__ status,
                                                          const int64_t *__restrict__ row_ptr,
                                                          const uint32_t *__restrict__ counts, int32_t *__restrict__ cols,
-                                                         unsigned long long col_cap)
+                                                         unsigned long long col_cap, const JobDesc *__restrict__ all_jobs,
+                                                         int nall, Report to)
 {
     __shared__ uint16_t list[kBandRows / 32][kListMax];
     __shared__ int64_t run[kBandRows / 32][32];  // where list entry 0 would go if it were lane l's
+    if (blockIdx.x == 0 && to.host_flags)  // null: scatter_records reports
+        report(to, row_ptr, all_jobs, nall);
     if (*hits > col_cap || *status != kStatusOk)
         return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1311,39 +1437,37 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         return s;
     if ((s = ensure(ctx, ctx->counts, (size_t)B.counts * sizeof(uint32_t), "segment counts")) != IG_OK)
         return s;
-    if ((s = ensure(ctx, ctx->flags, 8 * sizeof(unsigned long long), "flags")) != IG_OK)
+    if ((s = ensure(ctx, ctx->flags, kFlagWords * sizeof(unsigned long long), "flags")) != IG_OK)
         return s;
     // the scan workspace is sized here: nothing allocates inside a capture
-    const int64_t m = out ? (int64_t)out->n + 1 : 0;
-    if (out && (s = ensure(ctx, ctx->scan_tmp, (size_t)((m + kScanChunk - 1) / kScanChunk) * sizeof(int64_t),
+    const int64_t row_blocks = out ? ((int64_t)out->n + kPrefixRows - 1) / kPrefixRows : 0;
+    if (out && (s = ensure(ctx, ctx->scan_tmp, (size_t)(row_blocks + 1) * sizeof(unsigned long long),
                            "scan workspace")) != IG_OK)
         return s;
-    // job buffer: all jobs | job-boundary offsets (compaction) | pair_levels jobs | pair_deltas jobs | dense jobs
+    // job buffer: all jobs | pair_levels jobs | pair_deltas jobs | dense jobs
     const size_t jbytes = B.desc.size() * sizeof(JobDesc);
     const size_t bbytes = (B.desc.size() + 1) * sizeof(int64_t);
     const size_t nbytes = B.desc_levels.size() * sizeof(JobDesc), gbytes = B.desc_deltas.size() * sizeof(JobDesc);
     const size_t dbytes = out ? B.desc_dense.size() * sizeof(JobDesc) : 0;
-    const size_t table = jbytes + bbytes + nbytes + gbytes + dbytes;
+    const size_t table = jbytes + nbytes + gbytes + dbytes;
     if ((s = ensure(ctx, ctx->jobs, table, "job table")) != IG_OK)
         return s;
-    // staging: the job table image | 4 flag words read back | job bounds read back
+    // staging: the job table image | 4 flag words and the job bounds, written by the pass
     const size_t flag_off = (table + 63) & ~size_t(63), bound_off = flag_off + 64;
     if ((s = ensure_stage(ctx, bound_off + bbytes)) != IG_OK)
         return s;
     char *stage = static_cast<char *>(ctx->stage);
     std::memcpy(stage, B.desc.data(), jbytes);
-    std::memset(stage + jbytes, 0, bbytes);
     if (nbytes)
-        std::memcpy(stage + jbytes + bbytes, B.desc_levels.data(), nbytes);
+        std::memcpy(stage + jbytes, B.desc_levels.data(), nbytes);
     if (gbytes)
-        std::memcpy(stage + jbytes + bbytes + nbytes, B.desc_deltas.data(), gbytes);
+        std::memcpy(stage + jbytes + nbytes, B.desc_deltas.data(), gbytes);
     if (dbytes)
-        std::memcpy(stage + jbytes + bbytes + nbytes + gbytes, B.desc_dense.data(), dbytes);
+        std::memcpy(stage + jbytes + nbytes + gbytes, B.desc_dense.data(), dbytes);
     unsigned long long *host_flags = reinterpret_cast<unsigned long long *>(stage + flag_off);
     int64_t *host_bounds = reinterpret_cast<int64_t *>(stage + bound_off);
     char *jbase = static_cast<char *>(ctx->jobs.ptr);
     const JobDesc *d_jobs = reinterpret_cast<const JobDesc *>(jbase);
-    int64_t *d_bounds = reinterpret_cast<int64_t *>(jbase + jbytes);
     const int njobs = (int)B.desc.size();
     unsigned long long *flags = static_cast<unsigned long long *>(ctx->flags.ptr);
     PairArgs a;
@@ -1382,6 +1506,10 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         out ? (uint64_t)out->col_cap : 0, (uint64_t)a.wait_cycles, (uint64_t)a.skip_first_copy,
         (uint64_t)bits_bytes, (uint64_t)B.items_dense, dbytes, (uint64_t)(B.record_pairs > 0)};
     ctx->fault_tile_copy = false;  // the injected fault is one-shot
+    const PassZero zero{flags, out ? out->row_ptr : nullptr,
+                        out ? static_cast<unsigned long long *>(ctx->scan_tmp.ptr) : nullptr,
+                        out ? (long long)row_blocks + 1 : 0};
+    const Report to{flags, host_flags, host_bounds, n};
     int64_t launched = 0;
     s = run_graph(ctx, out ? 0 : 1, sig, out ? "build pass" : "count pass", [&]() -> cudaError_t {
         launched = 0;
@@ -1390,18 +1518,17 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
             return e;
         phase_begin(ctx, IG_PHASE_PREP);
         if (B.units > 0) {
-            prep_units<<<prep_grid, 256, 0, st>>>(d_words, d_jobs, njobs, B.units, static_cast<uint4 *>(ctx->sel.ptr));
+            prep_units<<<prep_grid, 256, 0, st>>>(d_words, d_jobs, njobs, B.units, static_cast<uint4 *>(ctx->sel.ptr),
+                                                   zero);
             launched++;
         }
         phase_end(ctx, IG_PHASE_PREP);
         if ((e = cudaGetLastError()) != cudaSuccess)
             return e;
-        if ((e = cudaMemsetAsync(flags, 0, 8 * sizeof(unsigned long long), st)) != cudaSuccess)
-            return e;
         phase_begin(ctx, IG_PHASE_PAIRS);
         PairArgs k = a;
         if (B.items_deltas > 0) {
-            k.jobs = reinterpret_cast<const JobDesc *>(jbase + jbytes + bbytes + nbytes);
+            k.jobs = reinterpret_cast<const JobDesc *>(jbase + jbytes + nbytes);
             k.njobs = (int)B.desc_deltas.size();
             k.items = B.items_deltas;
             pair_deltas<<<grid, kBandRows, 0, st>>>(k);
@@ -1410,7 +1537,7 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
                 return e;
         }
         if (B.items_levels > 0) {
-            k.jobs = reinterpret_cast<const JobDesc *>(jbase + jbytes + bbytes);
+            k.jobs = reinterpret_cast<const JobDesc *>(jbase + jbytes);
             k.njobs = (int)B.desc_levels.size();
             k.items = B.items_levels;
             k.work = flags + 4;
@@ -1421,49 +1548,37 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         }
         phase_end(ctx, IG_PHASE_PAIRS);
         if (out) {
-            if ((e = cudaMemsetAsync(out->row_ptr, 0, sizeof(int64_t), st)) != cudaSuccess)
-                return e;
             phase_begin(ctx, IG_PHASE_COMPACT);
             phase_begin(ctx, IG_PHASE_PREFIX);
-            row_prefix<<<(unsigned)((n + kPrefixRows - 1) / kPrefixRows), 256, 0, st>>>(
-                static_cast<uint32_t *>(ctx->counts.ptr), d_jobs, njobs, n, out->row_ptr);
+            row_offsets<<<(unsigned)row_blocks, 256, 0, st>>>(static_cast<uint32_t *>(ctx->counts.ptr), d_jobs, njobs, n,
+                                                              out->row_ptr, zero.scan_words, a.status, a.wait_cycles);
             launched++;
             if ((e = cudaGetLastError()) != cudaSuccess)
                 return e;
             phase_end(ctx, IG_PHASE_PREFIX);
-            // inclusive scan over row_ptr[0..n] (row_ptr[0] = 0) gives the offsets
-            phase_begin(ctx, IG_PHASE_SCAN);
-            if (inclusive_scan_i64(ctx, out->row_ptr, m) != IG_OK)
-                return cudaErrorLaunchFailure;
-            phase_end(ctx, IG_PHASE_SCAN);
             phase_begin(ctx, IG_PHASE_SCATTER);
             if (B.record_pairs > 0) {
                 scatter_records<<<sgrid, 256, 0, st>>>(a.rec, flags + 1, a.status, cap, d_jobs, njobs,
                                                         (unsigned long long)B.counts, out->row_ptr,
                                                         static_cast<const uint32_t *>(ctx->counts.ptr), out->cols,
-                                                        out->col_cap);
+                                                        out->col_cap, to);
                 launched++;
                 if ((e = cudaGetLastError()) != cudaSuccess)
                     return e;
             }
             if (B.items_dense > 0) {
                 expand_bits<<<(unsigned)B.items_dense, kBandRows, 0, st>>>(
-                    a.bits, reinterpret_cast<const JobDesc *>(jbase + jbytes + bbytes + nbytes + gbytes),
+                    a.bits, reinterpret_cast<const JobDesc *>(jbase + jbytes + nbytes + gbytes),
                     (int)B.desc_dense.size(), a.hit_count, a.status, out->row_ptr,
-                    static_cast<const uint32_t *>(ctx->counts.ptr), out->cols, out->col_cap);
+                    static_cast<const uint32_t *>(ctx->counts.ptr), out->cols, out->col_cap, d_jobs, njobs,
+                    B.record_pairs > 0 ? Report{} : to);
                 launched++;
                 if ((e = cudaGetLastError()) != cudaSuccess)
                     return e;
             }
             phase_end(ctx, IG_PHASE_SCATTER);
             phase_end(ctx, IG_PHASE_COMPACT);
-            job_bounds<<<(unsigned)((njobs + 1 + 255) / 256), 256, 0, st>>>(out->row_ptr, d_jobs, njobs, n,
-                                                                             d_bounds);
-            launched++;
-            if ((e = cudaGetLastError()) != cudaSuccess)
-                return e;
-            if ((e = cudaMemcpyAsync(host_bounds, d_bounds, bbytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-                return e;
+            return cudaSuccess;
         }
         return cudaMemcpyAsync(host_flags, flags, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
     });
