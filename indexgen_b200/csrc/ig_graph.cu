@@ -32,6 +32,7 @@
 #include <cstring>
 
 #include "ig_internal.h"
+#include "ig_pairs.cuh"
 #include "ig_slice.cuh"
 
 namespace ig {
@@ -41,57 +42,6 @@ namespace {
 using slice::imad;
 using slice::kUnitCols;
 using slice::Words2;
-
-constexpr unsigned kFull = 0xffffffffu;
-
-// Pass status word: a bounded wait ran out (the CTA left after its copies in
-// flight had landed), or, worse, a copy in flight never landed either.
-enum : int { kStatusOk = 0, kStatusTimeout = 1, kStatusCopyLost = 2 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_fence_init()
-{
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// 1-D TMA bulk copy global -> this CTA's shared memory (16-byte aligned,
-// size a multiple of 16).  Plain copy: no cluster multicast.
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
 
 // Index of the job whose `key` range contains v (jobs sorted by key).
 __device__ __forceinline__ int find_job_by_item(const JobDesc *jobs, int njobs, long long v)
@@ -200,73 +150,6 @@ __shared__ __align__(128) uint4 g_tile[2][kSlotVec];
 __shared__ __align__(8) uint64_t g_bar[2];
 __shared__ PairArgs g_args;
 __shared__ long long g_item;
-
-// Record slots.  Each warp takes slots from the global counter in chunks of
-// kSlotChunk (one atomic per chunk instead of one per hit group: a single
-// counter address is otherwise the limit on dense graphs) and keeps the rest
-// of its chunk, the same in every lane's registers.  Slots a warp never fills
-// are written as sentinels (cell = kNoCell) when the kernel ends; the scatter
-// skips them.
-constexpr unsigned kSlotChunk = 64;
-constexpr uint32_t kNoCell = 0xffffffffu;
-
-struct WarpSlots {
-    unsigned long long base;  // next free slot of the warp's chunk
-    unsigned left;            // free slots left in it
-};
-
-// Slots of the warp's next `total` records (warp-uniform call): record j goes
-// to b0 + j for j < n0, else to b1 + j (b1 already less n0).
-struct Slots {
-    unsigned long long b0, b1;
-    unsigned n0;
-};
-
-__device__ __forceinline__ Slots take_slots(WarpSlots &w, unsigned total, int lane)
-{
-    Slots s;
-    s.b0 = w.base;
-    s.b1 = 0;
-    s.n0 = total;
-    if (w.left >= total) {
-        w.base += total;
-        w.left -= total;
-        return s;
-    }
-    s.n0 = w.left;
-    const unsigned need = total - w.left;
-    const unsigned take = need > kSlotChunk ? need : kSlotChunk;
-    unsigned long long b1 = 0;
-    if (lane == 0)
-        b1 = atomicAdd(g_args.rec_count, (unsigned long long)take);
-    b1 = __shfl_sync(kFull, b1, 0);
-    s.b1 = b1 - s.n0;
-    w.base = b1 + need;
-    w.left = take - need;
-    return s;
-}
-
-// Warp total of cnt and this lane's exclusive prefix.  When no lane has more
-// than one hit (the usual case on sparse graphs) one ballot gives both,
-// otherwise a shuffle scan does.
-__device__ __forceinline__ void warp_count_prefix(uint32_t cnt, int lane, unsigned &total, unsigned &pre)
-{
-    const unsigned some = __ballot_sync(kFull, cnt != 0u);
-    if (__all_sync(kFull, cnt <= 1u)) {
-        total = (unsigned)__popc(some);
-        pre = (unsigned)__popc(some & ((1u << lane) - 1u));
-        return;
-    }
-    unsigned incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned t = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o)
-            incl += t;
-    }
-    total = __shfl_sync(kFull, incl, 31);
-    pre = incl - cnt;
-}
 
 // Thread 0: copy the tile of units starting at column c0 (at most kTileCols
 // columns, up to c_hi) into ring slot `slot`.
@@ -556,7 +439,7 @@ __device__ __noinline__ LoopState run_item(const JobDesc *job, int band, int seg
                 warp_count_prefix(cnt, lane, total, j);
                 if (total == 0u)
                     continue;
-                const Slots sl = take_slots(state.ws, total, lane);
+                const Slots sl = take_slots(now(g_args.rec_count), state.ws, total, lane);
                 const uint32_t cell = now(g_it.cell) + (uint32_t)tid;
                 const uint32_t off = (uint32_t)(col0 - now(g_it.seg0));
                 EdgeRecord *rec = now(g_args.rec);
@@ -729,44 +612,6 @@ __global__ void __launch_bounds__(kBandRows, 2) pair_deltas(PairArgs a) { pair_l
 // kernels' and ends in the same status.
 constexpr int kPrefixParts = 4;
 constexpr int kPrefixRows = 256 / kPrefixParts;
-constexpr unsigned long long kOwnSum = 1ull << 62, kPrefixSum = 2ull << 62, kSumMask = (1ull << 62) - 1;
-
-// Sum of the degrees of all blocks before block b; lane-parallel in one warp.
-// False when the wait ran out.
-__device__ __forceinline__ bool look_back(const unsigned long long *words, int64_t b, long long wait_cycles,
-                                          int *status, unsigned long long &before)
-{
-    const int lane = threadIdx.x & 31;
-    before = 0ull;
-    const long long t0 = clock64();
-    for (int64_t end = b; end > 0; end -= 32) {
-        const int64_t i = end - 1 - lane;
-        unsigned long long w = kPrefixSum;  // before block 0: an empty prefix
-        for (;;) {
-            if (i >= 0)
-                w = *reinterpret_cast<const volatile unsigned long long *>(words + i);
-            if (__all_sync(kFull, w != 0ull))
-                break;
-            // every lane sees lane 0's view of the clock and of the status
-            const bool stop = clock64() - t0 > wait_cycles ||
-                              *reinterpret_cast<const volatile int *>(status) != kStatusOk;
-            if (__shfl_sync(kFull, (int)stop, 0))
-                return false;
-        }
-        const unsigned full = __ballot_sync(kFull, (w & kPrefixSum) != 0ull);
-        // lanes up to the nearest complete prefix count
-        const int last = full != 0u ? __ffs(full) - 1 : 31;
-        unsigned long long v = lane <= last ? (w & kSumMask) : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v += __shfl_xor_sync(kFull, v, o);
-        before += v;
-        if (full != 0u)
-            break;
-    }
-    return true;
-}
-
 __global__ void __launch_bounds__(256) row_offsets(uint32_t *__restrict__ counts, const JobDesc *__restrict__ jobs,
                                                    int njobs, int64_t rows, int64_t *__restrict__ out,
                                                    unsigned long long *__restrict__ words, int *status,
@@ -1587,13 +1432,8 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         return s;
     IG_CUDA(cudaStreamSynchronize(st));
     phase_collect(ctx);
-    const int status = static_cast<int>(host_flags[2] & 0xffffffffu);
-    if (status == kStatusTimeout)
-        return set_error(ctx, IG_ERR_TIMEOUT, "pair kernel: a staged tile did not arrive within the wait limit");
-    if (status == kStatusCopyLost)
-        return set_error(ctx, IG_ERR_TIMEOUT,
-                         "pair kernel: a staged tile did not arrive within the wait limit, and a copy still in flight "
-                         "did not land either");
+    if ((s = pass_status(ctx, static_cast<int>(host_flags[2] & 0xffffffffu))) != IG_OK)
+        return s;
     *slots = host_flags[1];
     *hits = host_flags[3];
     if (bounds)
@@ -1633,6 +1473,19 @@ ig_status inclusive_scan_i64(Ctx *ctx, int64_t *x, int64_t m)
     IG_CUDA(cudaGetLastError());
     return IG_OK;
 }
+
+ig_status pass_status(Ctx *ctx, int status)
+{
+    if (status == kStatusTimeout)
+        return set_error(ctx, IG_ERR_TIMEOUT, "pair kernel: a staged tile did not arrive within the wait limit");
+    if (status == kStatusCopyLost)
+        return set_error(ctx, IG_ERR_TIMEOUT,
+                         "pair kernel: a staged tile did not arrive within the wait limit, and a copy still in flight "
+                         "did not land either");
+    return IG_OK;
+}
+
+ig_status ensure_staging(Ctx *ctx, size_t bytes) { return ensure_stage(ctx, bytes); }
 
 ig_status ensure_buffer(Ctx *ctx, DevBuf &b, size_t bytes, const char *what) { return ensure(ctx, b, bytes, what); }
 
@@ -1726,7 +1579,10 @@ PairPlan make_plan(int32_t n, long long target_items)
     return p;
 }
 
-ig_status count_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, int64_t *edges)
+namespace {
+
+// `general`: by the general pass whatever the jobs (the work split is timed on it).
+ig_status count_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, bool general, int64_t *edges)
 {
     ig_status s = check_jobs(ctx, jobs);
     if (s != IG_OK)
@@ -1740,11 +1596,21 @@ ig_status count_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         return IG_OK;
     }
     unsigned long long slots = 0, hits = 0;
-    s = run_pass(ctx, d_words, B, grid, nullptr, &slots, &hits, nullptr);
+    if (!general && jobs.size() == 1 && prefix_job(jobs[0]))
+        s = prefix_pass(ctx, d_words, jobs[0], nullptr, &slots, &hits, nullptr);
+    else
+        s = run_pass(ctx, d_words, B, grid, nullptr, &slots, &hits, nullptr);
     if (s != IG_OK)
         return s;
     *edges = (int64_t)hits;
     return IG_OK;
+}
+
+}  // namespace
+
+ig_status count_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, int64_t *edges)
+{
+    return count_jobs(ctx, d_words, jobs, false, edges);
 }
 
 // Work-split autotuner.  The pair kernels walk (256-row band x segment) item
@@ -1799,11 +1665,11 @@ ig_status autotune(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec>
         for (size_t k = 0; k < cands.size() && s == IG_OK; ++k) {
             ctx->items_per_cta[mode] = cands[k];
             if (k == 0)
-                s = count_batch(ctx, d_words, jobs, &edges);  // warm-up: workspaces grow here
+                s = count_jobs(ctx, d_words, jobs, true, &edges);  // warm-up: workspaces grow here
             float ms = 1e30f;
             for (int rep = 0; rep < 2 && s == IG_OK; ++rep) {
                 cudaEventRecord(e0, ctx->stream);
-                s = count_batch(ctx, d_words, jobs, &edges);
+                s = count_jobs(ctx, d_words, jobs, true, &edges);
                 cudaEventRecord(e1, ctx->stream);
                 const cudaError_t e = cudaEventSynchronize(e1);
                 float t = 0.f;
@@ -1876,6 +1742,11 @@ ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<Job
     return IG_OK;
 }
 
+// Edges per word beyond which a prefix build is done over by the general pass:
+// its rows come out unsorted, and rows of more than 256 columns are sorted one
+// CTA at a time.  (Uniform words reach 92 in the largest code workload.)
+constexpr unsigned long long kPrefixMaxDegree = 256;
+
 ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, Graph *g)
 {
     cudaStream_t st = ctx->stream;
@@ -1913,6 +1784,9 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         if (s != IG_OK)
             return s;
     }
+    // A lone large sparse job runs its shared prefixes once, unless it turns out
+    // to have so many edges that sorting its rows would cost more than that saves.
+    bool prefix = jobs.size() == 1 && !dense_job(jobs[0]) && prefix_job(jobs[0]);
     unsigned long long slots = 0, total = 0;
     for (int attempt = 0;; ++attempt) {
         // columns go to a context workspace with room for every record slot
@@ -1930,9 +1804,24 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         out.cols = static_cast<int32_t *>(ctx->cols_ws.ptr);
         out.col_cap = ctx->cols_ws.bytes / sizeof(int32_t);
         out.n = n;
-        s = run_pass(ctx, d_words, B, grid, &out, &slots, &total, g->job_edge_off.data());
+        if (prefix) {
+            const PrefixOut po{out.row_ptr, out.cols, out.col_cap};
+            s = prefix_pass(ctx, d_words, jobs[0], &po, &slots, &total, g->job_edge_off.data());
+        } else {
+            s = run_pass(ctx, d_words, B, grid, &out, &slots, &total, g->job_edge_off.data());
+        }
         if (s != IG_OK)
             return s;
+        const size_t tails = ((size_t)grid + (size_t)ctx->pair_grid_levels) * (kBandRows / 32) * kSlotChunk;
+        if (prefix && total > kPrefixMaxDegree * (unsigned long long)n) {
+            prefix = false;
+            attempt = -1;
+            ctx->col_room = std::max(ctx->col_room, total + total / 8);
+            const size_t want = (size_t)(total + total / 8) + tails + 1024;
+            if ((s = ensure(ctx, ctx->records, want * sizeof(EdgeRecord), "edge records")) != IG_OK)
+                return s;
+            continue;
+        }
         const unsigned long long record_cap = rec_capacity(ctx) - bits_bytes / sizeof(EdgeRecord);
         if (slots <= record_cap && total <= out.col_cap)
             break;
@@ -1942,7 +1831,6 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         if (slots > record_cap) {
             // slots of a rerun differ from this pass only by the chunk tails
             // of the warps (scheduling), so leave room for all of them
-            const size_t tails = ((size_t)grid + (size_t)ctx->pair_grid_levels) * (kBandRows / 32) * kSlotChunk;
             const size_t want = (size_t)(slots + slots / 8) + tails + 1024;
             s = ensure(ctx, ctx->records, bits_bytes + want * sizeof(EdgeRecord), "edge records");
             if (s != IG_OK)

@@ -249,6 +249,30 @@ ig_status autotune(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec>
 // tests).  Caller holds ctx->mu.
 ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs);
 
+// The pair pass of one large sparse job with shared prefixes run once
+// (ig_prefix.cu).  prefix_job: jobs it takes.  A build (`out` set) leaves the
+// upper CSR; *slots > record capacity or *hits > col_cap: void, as for the
+// general pass.
+constexpr int kPrefixMinLen = 10;
+// From here on it wins at every length and threshold it takes: a build of
+// 28,000 words took 137 us against 138 at L = 13, k = 2 and 261 against 276 at
+// L = 16, k = 4, one of 36,000 words 166 against 195 and 358 against 420;
+// with 20,000 words the general pass is faster.
+constexpr int32_t kPrefixMinWords = 32768;
+constexpr int32_t kPrefixLongWords = 131072;  // prefixes of 8 characters instead of 7
+struct PrefixOut {
+    int64_t *row_ptr = nullptr;
+    int32_t *cols = nullptr;
+    unsigned long long col_cap = 0;
+};
+bool prefix_job(const JobSpec &j);
+ig_status prefix_pass(Ctx *ctx, const uint32_t *d_words, const JobSpec &job, const PrefixOut *out,
+                      unsigned long long *slots, unsigned long long *hits, int64_t *bounds);
+// Status word of a finished pair pass as a status with its message, and
+// page-locked staging of at least `bytes` on an idle context stream (ig_graph.cu).
+ig_status pass_status(Ctx *ctx, int status);
+ig_status ensure_staging(Ctx *ctx, size_t bytes);
+
 // In-place inclusive scan of m int64 on the context stream (ig_graph.cu).
 ig_status inclusive_scan_i64(Ctx *ctx, int64_t *x, int64_t m);
 ig_status ensure_buffer(Ctx *ctx, DevBuf &b, size_t bytes, const char *what);

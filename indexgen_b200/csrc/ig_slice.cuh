@@ -138,22 +138,28 @@ __host__ __device__ __forceinline__ uint32_t level_step(bool all, uint32_t prev,
                                                                    : or3(and_or(prev, m, x), y, z);
 }
 
-// S[0][k](L) by levels.  eq(i, j): the columns whose character at j equals
-// the row's at i.  For k = 0 and 1 (K = 1) `k0` is 0 or all ones: hits at
-// distance 1 only count when it is set.
-template <int L, int K, class Eq>
-__host__ __device__ __forceinline__ Words2 levels(const Eq &eq, uint32_t k0)
+// The level words S[t + W][e] of a row's prefix.
+template <int K>
+using Levels = Words2[2 * (K / 2) + 1][K + 1];
+
+template <int K>
+__host__ __device__ __forceinline__ void levels_start(Levels<K> &S)
 {
-    constexpr int W = K / 2;
-    constexpr uint32_t kAll = 0xffffffffu;
-    Words2 S[2 * W + 1][K + 1];
     IG_UNROLL
-    for (int t = 0; t < 2 * W + 1; ++t)
+    for (int t = 0; t < 2 * (K / 2) + 1; ++t)
         IG_UNROLL
         for (int e = 0; e <= K; ++e)
-            S[t][e] = Words2{kAll, kAll};
+            S[t][e] = Words2{0xffffffffu, 0xffffffffu};
+}
+
+// S from the prefix of I0 characters to that of I1.  eq(i, j): the columns
+// whose character at j equals the row's at i.
+template <int L, int K, int I0, int I1, class Eq>
+__host__ __device__ __forceinline__ void levels_advance(const Eq &eq, Levels<K> &S)
+{
+    constexpr int W = K / 2;
     IG_UNROLL
-    for (int i = 1; i <= L; ++i) {
+    for (int i = I0 + 1; i <= I1; ++i) {
         IG_UNROLL
         for (int t = -W; t <= W; ++t) {
             const int j = i + t;
@@ -191,10 +197,20 @@ __host__ __device__ __forceinline__ Words2 levels(const Eq &eq, uint32_t k0)
             }
         }
     }
-    Words2 r = S[W][K];
+}
+
+// The hits S[0][k](L).  For k = 0 and 1 (K = 1) `k0` is 0 or all ones: hits at
+// distance 1 only count when it is set.
+template <int L, int K, class Eq>
+__host__ __device__ __forceinline__ Words2 levels(const Eq &eq, uint32_t k0)
+{
+    Levels<K> S;
+    levels_start<K>(S);
+    levels_advance<L, K, 0, L>(eq, S);
+    Words2 r = S[K / 2][K];
     if (K == 1) {
-        r.a &= S[W][0].a | k0;
-        r.b &= S[W][0].b | k0;
+        r.a &= S[K / 2][0].a | k0;
+        r.b &= S[K / 2][0].b | k0;
     }
     return r;
 }
