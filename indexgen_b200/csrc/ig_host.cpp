@@ -210,17 +210,17 @@ class BucketGreedy {
     // ap covers the n job rows (its differences are the degrees); neighbour
     // ids in the rows are global and `base` maps them to job-local ids.
     BucketGreedy(const int64_t *ap, Rows rows, int32_t n, int64_t base)
-        : ap_(ap), rows_(rows), base_(base), v_((size_t)n)
+        : ap_(ap), rows_(rows), base_(base), deg_((size_t)n), pos_((size_t)n)
     {
         int32_t maxd = 0;
         for (int32_t i = 0; i < n; ++i) {
-            v_[(size_t)i].deg = (int32_t)(ap[i + 1] - ap[i]);
-            maxd = std::max(maxd, v_[(size_t)i].deg);
+            deg_[(size_t)i] = (int32_t)(ap[i + 1] - ap[i]);
+            maxd = std::max(maxd, deg_[(size_t)i]);
         }
         nb_ = maxd + 1;
         std::vector<int64_t> hist((size_t)nb_ + 1, 0);
         for (int32_t i = 0; i < n; ++i)
-            hist[(size_t)v_[(size_t)i].deg]++;
+            hist[(size_t)deg_[(size_t)i]]++;
         // cap_b = #{v : deg >= b}
         start_.resize((size_t)nb_ + 1);
         size_.assign((size_t)nb_, 0);
@@ -234,20 +234,30 @@ class BucketGreedy {
         data_.reset(new int32_t[(size_t)std::max<int64_t>(off, 1)]);
         tracker_ = maxd + 1;
         for (int32_t i = 0; i < n; ++i) {  // RowsBySum: ascending vertex id
-            const int32_t d = v_[(size_t)i].deg;
-            v_[(size_t)i].pos = size_[(size_t)d];
+            const int32_t d = deg_[(size_t)i];
+            pos_[(size_t)i] = size_[(size_t)d];
             data_[(size_t)(start_[(size_t)d] + size_[(size_t)d]++)] = i;
             tracker_ = std::min(tracker_, d);
         }
         active_ = n;
-        todel_.reserve((size_t)maxd + 1);
+        todel_.resize((size_t)maxd + 1);
         bufx_.resize((size_t)maxd + 1);
         bufi_.resize((size_t)maxd + 1);
+        moves_.reset(new Move[(size_t)kMoves]);
     }
 
+    // One ball at a time: first all its rows are walked, which lowers the
+    // degrees and lists the bucket moves (vertex, old degree) without a branch
+    // on whether a neighbour is live; then the moves are applied in that order.
+    // The walk reads and writes degrees only and the moves touch buckets and
+    // positions only, so every bucket sees the sequence of appends and
+    // swap-removals that walking and moving in turn would give it.  (Against
+    // testing each neighbour and moving it at once: 5.12 -> 3.83 ms on 744,076
+    // entries of 30,000 words, 21.4 -> 15.2 on 4.5 million of 10,000.)
     int32_t run(int32_t *order)
     {
         int32_t cnt = 0;
+        int32_t *deg = deg_.data();
         while (active_ > 0) {
             // MinSumRow: back of the minimum bucket
             const int32_t x = data_[(size_t)(start_[(size_t)tracker_] + size_[(size_t)tracker_] - 1)];
@@ -255,98 +265,100 @@ class BucketGreedy {
             // DelBall: active neighbours in m-order, then the vertex itself
             const int32_t *row = rows_.get(x, bufx_.data());
             const int64_t len = ap_[x + 1] - ap_[x];
-            todel_.resize((size_t)len + 1);
             int32_t nt = 0;
             for (int64_t k = 0; k < len; ++k) {  // branch-free compaction
                 const int32_t j = (int32_t)(row[k] - base_);
                 todel_[(size_t)nt] = j;
-                nt += v_[(size_t)j].deg >= 0;
+                nt += deg[j] >= 0;
             }
             todel_[(size_t)nt++] = x;
             // the neighbour lists of the ball's vertices are read next: fetch
             // their heads a few vertices ahead
             for (int32_t t = 0; t < nt && t < 4; ++t)
                 rows_.prefetch(todel_[(size_t)t]);
+            int32_t m = 0;  // moves listed
             for (int32_t t = 0; t < nt; ++t) {
                 if (t + 4 < nt)
                     rows_.prefetch(todel_[(size_t)t + 4]);
-                del_row_col(todel_[(size_t)t]);
+                const int32_t i = todel_[(size_t)t];
+                const int32_t *ri = rows_.get(i, bufi_.data());
+                const int64_t e = ap_[i + 1] - ap_[i];
+                for (int64_t k0 = 0; k0 < e; k0 += kChunk) {
+                    const int64_t k1 = std::min<int64_t>(e, k0 + kChunk);
+                    if (m + (k1 - k0) >= kMoves) {
+                        apply(m);
+                        m = 0;
+                    }
+                    for (int64_t k = k0; k < k1; ++k) {
+                        const int32_t j = (int32_t)(ri[k] - base_);
+                        const int32_t d = deg[j];
+                        moves_[m].v = j;
+                        moves_[m].cur = d;
+                        deg[j] = d - (d > 0);
+                        m += d > 0;
+                    }
+                }
+                moves_[m].v = i;  // the vertex goes: a move to nowhere
+                moves_[m].cur = deg[i] | kDelete;
+                if (++m == kMoves) {
+                    apply(m);
+                    m = 0;
+                }
+                deg[i] = -1;
+                --active_;
             }
+            apply(m);
         }
         return cnt;
     }
 
   private:
-    void delete_row(int32_t cur, int32_t row)
-    {
-        const int64_t base = start_[(size_t)cur];
-        const int32_t sz = --size_[(size_t)cur];
-        const int32_t p = v_[(size_t)row].pos;
-        const int32_t last = data_[(size_t)(base + sz)];
-        data_[(size_t)(base + p)] = last;
-        v_[(size_t)last].pos = p;
-        if (cur == tracker_ && sz == 0)
-            while (tracker_ < nb_ && size_[(size_t)tracker_] == 0)
-                ++tracker_;
-    }
+    static constexpr int kMoves = 8192, kChunk = 4096;
+    static constexpr int32_t kDelete = INT32_MIN;
 
-    void decrease_sum(int32_t cur, int32_t row)
+    // AdjList's DeleteRow, and DecreaseSum's append to the bucket below.
+    void apply(int32_t m)
     {
-        delete_row(cur, row);
-        const int32_t b = cur - 1;
-        const int32_t s = size_[(size_t)b]++;
-        data_[(size_t)(start_[(size_t)b] + s)] = row;
-        v_[(size_t)row].deg = b;
-        v_[(size_t)row].pos = s;
-        if (b < tracker_)
-            tracker_ = b;
-    }
-
-    // Neighbours are visited in blocks of 8: their degrees are loaded together
-    // (independent loads overlap, the next block's are prefetched) and only
-    // the live ones (degree > 0) are walked through a bitmask.  Exact: within one pass over m[i] the
-    // neighbours are distinct and decrease_sum(j) changes only deg[j].
-    void del_row_col(int32_t i)
-    {
-        const int32_t di = v_[(size_t)i].deg;
-        if (di < 0)
-            return;
-        const int32_t *row = rows_.get(i, bufi_.data());
-        const int64_t e = ap_[i + 1] - ap_[i];
-        for (int64_t k = 0; k < e; k += 8) {
-            const int m = (int)std::min<int64_t>(8, e - k);
-            for (int64_t q = k + 8; q < std::min<int64_t>(k + 16, e); ++q)  // next block's degrees
-                __builtin_prefetch(&v_[(size_t)(row[q] - base_)]);
-            int32_t jj[8], dd[8];
-            unsigned live = 0;
-            for (int t = 0; t < m; ++t) {
-                jj[t] = (int32_t)(row[k + t] - base_);
-                dd[t] = v_[(size_t)jj[t]].deg;
-            }
-            for (int t = 0; t < m; ++t)
-                live |= (unsigned)(dd[t] > 0) << t;
-            while (live) {
-                const int t = __builtin_ctz(live);
-                live &= live - 1;
-                decrease_sum(dd[t], jj[t]);
+        int32_t *pos = pos_.data(), *size = size_.data(), *data = data_.get();
+        const int64_t *start = start_.data();
+        int32_t tracker = tracker_;
+        for (int32_t c = 0; c < m; ++c) {
+            if (c + 8 < m)
+                __builtin_prefetch(pos + moves_[c + 8].v);
+            const int32_t v = moves_[c].v, cur = moves_[c].cur & ~kDelete;
+            const int64_t base = start[cur];
+            const int32_t s = --size[cur];
+            const int32_t q = pos[v];
+            const int32_t last = data[base + s];
+            data[base + q] = last;
+            pos[last] = q;
+            if (cur == tracker && s == 0)
+                while (tracker < nb_ && size[tracker] == 0)
+                    ++tracker;
+            if (moves_[c].cur >= 0) {
+                const int32_t b = cur - 1;
+                const int32_t s1 = size[b]++;
+                data[start[b] + s1] = v;
+                pos[v] = s1;
+                if (b < tracker)
+                    tracker = b;
             }
         }
-        delete_row(v_[(size_t)i].deg, i);
-        v_[(size_t)i].deg = -1;
-        --active_;
+        tracker_ = tracker;
     }
 
-    struct Vtx {
-        int32_t deg;  // current degree, -1 once deleted
-        int32_t pos;  // slot inside its degree bucket
+    struct Move {
+        int32_t v, cur;  // vertex, the degree it had (kDelete set: it goes)
     };
     const int64_t *ap_;
     Rows rows_;
     int64_t base_;
-    std::vector<Vtx> v_;
+    std::vector<int32_t> deg_;  // current degree, -1 once deleted
+    std::vector<int32_t> pos_;  // slot inside its degree bucket
     std::vector<int32_t> size_;
     std::vector<int64_t> start_;
     std::unique_ptr<int32_t[]> data_;
+    std::unique_ptr<Move[]> moves_;
     std::vector<int32_t> todel_, bufx_, bufi_;
     int32_t nb_ = 0;
     int32_t tracker_ = 0;
