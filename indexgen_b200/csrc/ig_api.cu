@@ -1166,6 +1166,15 @@ ig_status ig_graph_device_csr(const ig_graph *g, const int64_t **row_ptr, const 
     IG_ABI_TRY
     if (!g || !row_ptr || !cols)
         return IG_ERR_INPUT;
+    ig_graph *m = const_cast<ig_graph *>(g);
+    if (m->cols_pending) {
+        std::lock_guard<std::mutex> lk(g->ctx->mu);
+        ig::DeviceGuard dg(g->ctx->device);
+        const cudaError_t e = cudaStreamSynchronize(g->ctx->stream);
+        if (e != cudaSuccess)
+            return ig::cuda_error(g->ctx, e, "column copy");
+        m->cols_pending = false;
+    }
     *row_ptr = g->d_row_ptr;
     *cols = g->d_cols;
     return IG_OK;

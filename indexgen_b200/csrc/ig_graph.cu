@@ -94,12 +94,26 @@ struct PassZero {
     long long scan_count;
 };
 
+// A small job table travels as an argument of the first kernel, which writes it
+// to device memory for the others: a copy node before it would cost every
+// small build some 4 us.
+constexpr int kInlineVecs = 224;
+struct InlineTable {
+    uint4 v[kInlineVecs];
+    int vecs;  // 0: the table has been copied
+};
+static_assert(sizeof(JobDesc) % sizeof(uint4) == 0, "tables are whole vectors");
+
 // Column units of every job, one warp per unit of 64 columns: word (j, c, h)
 // has bit b set where column 32 h + b of the unit has character c at position j.
-__global__ void prep_units(const uint32_t *__restrict__ words, const JobDesc *__restrict__ jobs, int njobs,
-                           long long total_units, uint4 *__restrict__ units, PassZero zero)
+__global__ void prep_units(const uint32_t *__restrict__ words, JobDesc *__restrict__ table, int njobs,
+                           long long total_units, uint4 *__restrict__ units, PassZero zero,
+                           const __grid_constant__ InlineTable given)
 {
     const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const JobDesc *jobs = given.vecs > 0 ? reinterpret_cast<const JobDesc *>(given.v) : table;
+    for (int k = (int)id; k < given.vecs && id < kInlineVecs; k += kInlineVecs)
+        reinterpret_cast<uint4 *>(table)[k] = given.v[k];
     if (id < kFlagWords)
         zero.flags[id] = 0ull;
     if (zero.row_ptr && id == 0)
@@ -149,7 +163,7 @@ constexpr int kSlotVec = kTileCols / kUnitCols * slice::unit_vec(IG_MAX_LEN);  /
 __shared__ __align__(128) uint4 g_tile[2][kSlotVec];
 __shared__ __align__(8) uint64_t g_bar[2];
 __shared__ PairArgs g_args;
-__shared__ long long g_item;
+__shared__ long long g_item[2];  // the next item, alternating
 
 // Thread 0: copy the tile of units starting at column c0 (at most kTileCols
 // columns, up to c_hi) into ring slot `slot`.
@@ -288,6 +302,7 @@ struct DeltaForm {
 struct LoopState {
     WarpSlots ws;
     uint32_t parity;  // bit b: phase parity of ring slot b; kSkipped
+    int turn;         // items run so far, modulo 2
     bool aborted;
 };
 
@@ -367,6 +382,8 @@ __device__ __noinline__ LoopState run_item(const JobDesc *job, int band, int seg
             for (int t = 0; t < 2 && t < ntiles; ++t)
                 if (!(t == 0 && (state.parity & kSkipped)))
                     ring_issue<L>(t, g_it.units, c_lo + t * kTileCols, c_hi);
+            // the next item's number, while the tile is on its way
+            g_item[state.turn] = (long long)gridDim.x + (long long)atomicAdd(g_args.work, 1ull);
         }
     }
     const uint32_t one = g_args.one;
@@ -465,21 +482,22 @@ __device__ __noinline__ LoopState run_item(const JobDesc *job, int band, int seg
 // a band of group g owns segments g..nseg-1.  Every group before the last is
 // full, so group g starts at item bands_per_seg * (g * nseg - g (g - 1) / 2);
 // g is found by bisection.
-__device__ __forceinline__ void decode_item(const JobDesc &J, long long li, int &band, int &seg)
+__device__ __forceinline__ void decode_item(const JobDesc &J, long long local, int &band, int &seg)
 {
-    int lo = 0, hi = J.nseg - 1;
+    // a job has at most 65,536 bands x 256 segments: 32 bits
+    const uint32_t li = (uint32_t)local, nseg = (uint32_t)J.nseg, bps = (uint32_t)J.bands_per_seg;
+    uint32_t lo = 0, hi = nseg - 1;
     while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        const long long b = (long long)J.bands_per_seg * ((long long)mid * J.nseg - (long long)mid * (mid - 1) / 2);
-        if (b <= li)
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (bps * (mid * nseg - mid * (mid - 1) / 2) <= li)
             lo = mid;
         else
             hi = mid - 1;
     }
-    const long long q = li - (long long)J.bands_per_seg * ((long long)lo * J.nseg - (long long)lo * (lo - 1) / 2);
-    const int per = J.nseg - lo;
-    band = lo * J.bands_per_seg + (int)(q / per);
-    seg = lo + (int)(q % per);
+    const uint32_t q = li - bps * (lo * nseg - lo * (lo - 1) / 2);
+    const uint32_t per = nseg - lo;
+    band = (int)(lo * bps + q / per);
+    seg = (int)(lo + q % per);
 }
 
 // The unused rest of each warp's record-slot chunk becomes sentinels.
@@ -527,15 +545,12 @@ __device__ __forceinline__ void pair_loop(const PairArgs &args)
     st.ws.base = 0ull;
     st.ws.left = 0u;
     st.parity = 0u;
+    st.turn = 0;
     st.aborted = false;
 
-    for (;;) {
-        if (tid == 0)
-            g_item = (long long)atomicAdd(args.work, 1ull);
-        __syncthreads();
-        const long long item = g_item;
-        if (item >= args.items)
-            break;
+    // the first item by the CTA's number, the others from the counter, each
+    // fetched while the one before it is under way (run_item)
+    for (long long item = blockIdx.x; item < args.items; item = g_item[st.turn ^ 1]) {
         const JobDesc *J = args.jobs + find_job_by_item(args.jobs, args.njobs, item);
         int band = 0, seg = 0;
         decode_item(*J, item - J->item_off, band, seg);
@@ -568,7 +583,8 @@ __device__ __forceinline__ void pair_loop(const PairArgs &args)
 #undef IG_DELTAS
         if (st.aborted)
             break;
-        __syncthreads();
+        __syncthreads();  // the item is done with its shared values, and the next one's number is there
+        st.turn ^= 1;     // (the number after it goes to the other place: slow warps may still read this one)
     }
     if (st.aborted && tid == 0)
         ring_drain(st.parity);
@@ -1312,7 +1328,7 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     unsigned long long *host_flags = reinterpret_cast<unsigned long long *>(stage + flag_off);
     int64_t *host_bounds = reinterpret_cast<int64_t *>(stage + bound_off);
     char *jbase = static_cast<char *>(ctx->jobs.ptr);
-    const JobDesc *d_jobs = reinterpret_cast<const JobDesc *>(jbase);
+    JobDesc *d_jobs = reinterpret_cast<JobDesc *>(jbase);
     const int njobs = (int)B.desc.size();
     unsigned long long *flags = static_cast<unsigned long long *>(ctx->flags.ptr);
     PairArgs a;
@@ -1340,7 +1356,10 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     const int sgrid = (int)std::min<unsigned long long>(
         (std::min<unsigned long long>(cap, (unsigned long long)B.record_pairs) + 255) / 256 + 1,
         (unsigned long long)ctx->sm_count * 16);
-    const std::vector<uint64_t> sig = {
+    InlineTable given;
+    given.vecs = table <= sizeof(given.v) && B.units > 0 ? (int)(table / sizeof(uint4)) : 0;
+    std::memcpy(given.v, stage, given.vecs * sizeof(uint4));
+    std::vector<uint64_t> sig = {
         (uint64_t)(uintptr_t)stage,  table, (uint64_t)(uintptr_t)jbase, (uint64_t)(uintptr_t)d_words,
         (uint64_t)B.units,           (uint64_t)njobs, (uint64_t)(uintptr_t)ctx->sel.ptr,
         (uint64_t)(uintptr_t)flags,  (uint64_t)(uintptr_t)ctx->records.ptr, cap,
@@ -1350,6 +1369,11 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
         (uint64_t)sgrid,             (uint64_t)(uintptr_t)ctx->scan_tmp.ptr, (uint64_t)B.counts,
         out ? (uint64_t)out->col_cap : 0, (uint64_t)a.wait_cycles, (uint64_t)a.skip_first_copy,
         (uint64_t)bits_bytes, (uint64_t)B.items_dense, dbytes, (uint64_t)(B.record_pairs > 0)};
+    {  // an inline table is an argument too
+        const size_t at = sig.size();
+        sig.resize(at + given.vecs * 2);
+        std::memcpy(sig.data() + at, given.v, given.vecs * sizeof(uint4));
+    }
     ctx->fault_tile_copy = false;  // the injected fault is one-shot
     const PassZero zero{flags, out ? out->row_ptr : nullptr,
                         out ? static_cast<unsigned long long *>(ctx->scan_tmp.ptr) : nullptr,
@@ -1358,13 +1382,13 @@ ig_status run_pass(Ctx *ctx, const uint32_t *d_words, const BatchLayout &B, int 
     int64_t launched = 0;
     s = run_graph(ctx, out ? 0 : 1, sig, out ? "build pass" : "count pass", [&]() -> cudaError_t {
         launched = 0;
-        cudaError_t e = cudaMemcpyAsync(jbase, stage, table, cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess)
+        cudaError_t e = cudaSuccess;
+        if (given.vecs == 0 && (e = cudaMemcpyAsync(jbase, stage, table, cudaMemcpyHostToDevice, st)) != cudaSuccess)
             return e;
         phase_begin(ctx, IG_PHASE_PREP);
         if (B.units > 0) {
             prep_units<<<prep_grid, 256, 0, st>>>(d_words, d_jobs, njobs, B.units, static_cast<uint4 *>(ctx->sel.ptr),
-                                                   zero);
+                                                   zero, given);
             launched++;
         }
         phase_end(ctx, IG_PHASE_PREP);
@@ -1852,9 +1876,11 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
     }
     IG_CUDA(dev_malloc(ctx, (void **)&g->d_cols, std::max<size_t>((size_t)total, 1) * sizeof(int32_t), st));
     if (total > 0) {
+        // the copy is in order with everything the library does on the stream;
+        // only a caller that takes the raw pointers has to see it finished
         IG_CUDA(cudaMemcpyAsync(g->d_cols, ctx->cols_ws.ptr, (size_t)total * sizeof(int32_t), cudaMemcpyDeviceToDevice,
                                 st));
-        IG_CUDA(cudaStreamSynchronize(st));
+        g->cols_pending = true;
     }
     return IG_OK;
 }

@@ -159,8 +159,7 @@ void assemble(const int64_t *row_ptr, const int32_t *cols_in, int32_t n, int64_t
 // minimum tracker that only advances when the tracked bucket empties.
 //
 // Layout: the degree doubles as the deletion mark (-1 = deleted; the
-// reference skips deleted neighbours and neighbours of degree 0 alike) and
-// sits next to the bucket position of the same vertex; and
+// reference skips deleted neighbours and neighbours of degree 0 alike), and
 // all buckets share one flat array: bucket b gets a fixed slice of
 // #{v : initial degree >= b} slots, which bounds its size at any time because
 // degrees only fall.  The slice array is left uninitialised so only the slots

@@ -209,6 +209,7 @@ struct Graph {
     std::vector<int32_t> job_seg_shift, job_nseg;  // pair-pass tiling per job (0 when not built here)
     int64_t *d_row_ptr = nullptr;       // [n+1]
     int32_t *d_cols = nullptr;          // [edges], global column ids
+    std::atomic<bool> cols_pending{false};  // d_cols is still being copied on the context stream
     // host copies, filled on first use
     std::vector<int64_t> h_row_ptr;
     std::vector<int32_t> h_cols;
