@@ -16,7 +16,7 @@ coset vector, filtered (maxRun 3, GC [0.3,0.7]) to 207,432 words, editDist 4:
                into pinned memory (wall clock around the synchronous calls).
 * roofline  -- the pair-test kernel against the ALU-pipe peak (SMs x 64
                LOP3/PRMT lanes x max SM clock); algorithmic work = the ALU-pipe
-               ops the bit-sliced test needs (sliced_ops_per_pair),
+               ops the bit-sliced test needs (build_pass_of),
                measured traffic from the committed ncu summary.  The 16*L
                integer-op convention against the INT32 peak is reported beside
                it (int_ops_16L_convention).
@@ -288,7 +288,7 @@ def path_traffic_line(wl_name, edges: int, n: int):
     plan = 16 * edges + 20 * n
     return {"bytes_per_build": t, "bytes_per_edge": (t / edges) if t and edges else None,
             "plan_bytes_16E_20N": plan, "ratio_to_plan": (t / plan) if t else None,
-            "source": f"profiles/compaction_{wl_name}.md (ncu dram__bytes_read + write, pair kernel to scatter)"}
+            "source": f"profiles/compaction_{wl_name}.md (ncu dram__bytes_read + write, pair kernel to the finished columns)"}
 
 
 def touched_cells(n: int, seg_width: int, segments: int, band_rows: int = 256) -> int:
@@ -301,58 +301,73 @@ def touched_cells(n: int, seg_width: int, segments: int, band_rows: int = 256) -
     return int(np.sum(rows * np.maximum(segments - first, 0)))
 
 
+def level_ops(L: int, k: int, cuts) -> list:
+    """LOP3 operations per 32 pair tests of the level recurrence (ig_slice.cuh)
+    at threshold k, for the row positions (cuts[q], cuts[q + 1]] each: its
+    and/or terms as three-input operations, constants folded, only what
+    reaches the result."""
+    w = k // 2
+    nodes, at, one = [], [], "one"
+
+    def op(i, *ins):
+        nodes.append([x for x in ins if x != "match"])
+        at.append(i)
+        return len(nodes) - 1
+
+    def fold(i, prev, rest):  # (prev & match) | rest
+        if one in rest:
+            return one
+        acc = ["match"] + rest if prev == one else [op(i, prev, *rest[:1])] + rest[1:]
+        while len(acc) > 1:
+            acc = [op(i, *acc[:3])] + acc[3:]
+        return acc[0]
+
+    ok = lambda t, e: abs(t) <= w and abs(t) <= e <= k - abs(t)
+    S = {(t, e): one for t in range(-w, w + 1) for e in range(k + 1)}
+    for i in range(1, L + 1):
+        for t in range(-w, w + 1):
+            for e in range(k, -1, -1):
+                if 1 <= i + t <= L and ok(t, e) and e < max(i, i + t):
+                    S[t, e] = fold(i, S[t, e], [S[q] for q in ((t, e - 1), (t + 1, e - 1), (t - 1, e - 1)) if ok(*q)])
+    live, todo = set(), [S[0, k]]
+    while todo:
+        x = todo.pop()
+        if x not in live and not isinstance(x, str):
+            live.add(x)
+            todo += nodes[x]
+    return [sum(lo < at[x] <= hi for x in live) for lo, hi in zip(cuts, cuts[1:])]
+
+
 def sliced_ops_per_pair(L: int, d: int) -> float:
-    """LOP3 operations of the bit-sliced pair test (ig_slice.cuh) per pair
-    test.  Level form (editDist <= 5): the recurrence's and/or terms as
-    three-input operations, constants folded, only what reaches the result.
-    Delta form: 5 per band cell, 4 fewer per row, plus 2 per row for the
-    distance counter (not folded)."""
+    """LOP3 operations of the bit-sliced pair test per pair test: the level
+    form (editDist <= 5), or the delta form's 5 per band cell, 4 fewer per row,
+    plus 2 per row for the distance counter (not folded)."""
     k = d - 1
     if k >= L:  # every pair
         return 1 / 32
     if k < 2:  # mismatch levels only
         return (1 + k) * L / 32
-    w = k // 2
     if k > 4:
-        return L * (5 * (2 * w + 1) - 4 + 2) / 32
-    nodes, one, zero = [], "one", "zero"
+        return L * (5 * (2 * (k // 2) + 1) - 4 + 2) / 32
+    return level_ops(L, k, (0, L))[0] / 32
 
-    def op(*ins):
-        nodes.append([x for x in ins if x != "match"])
-        return len(nodes) - 1
 
-    def fold(prev, terms):  # (prev & match) | terms
-        if one in terms:
-            return one
-        rest = [t for t in terms if t != zero]
-        if prev == one:
-            acc = ["match"] + rest
-        elif prev == zero:
-            acc = rest
-        else:
-            acc = [op(prev, *rest[:1])] + rest[1:]
-        while len(acc) > 1:
-            acc = [op(*acc[:3])] + acc[3:]
-        return acc[0] if acc else zero
+PREFIX_MIN_WORDS, PREFIX_MIN_LEN, PREFIX_LONG_WORDS = 32768, 10, 131072  # ig_internal.h
 
-    ok = lambda t, e: abs(t) <= w and abs(t) <= e <= k - abs(t)
-    S = {(t, e): one if 0 <= t <= e else zero for t in range(-w, w + 1) for e in range(k + 1)}
-    for i in range(1, L + 1):
-        for t in range(-w, w + 1):
-            if i + t == 0:
-                S.update({(t, e): one if e >= -t else zero for e in range(k + 1)})
-            if not 1 <= i + t <= L:
-                continue
-            for e in range(k, -1, -1):
-                if ok(t, e):
-                    S[t, e] = fold(S[t, e], [S[q] for q in ((t, e - 1), (t + 1, e - 1), (t - 1, e - 1)) if ok(*q)])
-    live, todo = set(), [S[0, k]]
-    while todo:
-        x = todo.pop()
-        if x not in live and x != "match":
-            live.add(x)
-            todo += nodes[x]
-    return len(live) / 32
+
+def build_pass_of(words, L: int, d: int):
+    """(pair kernel, LOP3 operations per pair test) of a lone build of these
+    words: with shared prefixes (ig_prefix.cu) the levels of the first D1 and D2
+    characters run once per distinct prefix, not once per word."""
+    n = len(words)
+    if n < PREFIX_MIN_WORDS or L < PREFIX_MIN_LEN or not 3 <= d <= 5 or d >= L // 2:
+        return ("pair_levels" if d <= 5 else "pair_deltas"), sliced_ops_per_pair(L, d)
+    d2 = 8 if n >= PREFIX_LONG_WORDS else 7
+    d1 = d2 - 2
+    w = np.asarray(words, np.uint32)
+    share = [len(np.unique(w & np.uint32((1 << 2 * x) - 1))) / n for x in (d1, d2)]
+    ops = level_ops(L, d - 1, (0, d1, d2, L))
+    return "prefix_pairs", (ops[0] * share[0] + ops[1] * share[1] + ops[2]) / 32
 
 
 def alu_ops_per_pair(L: int, d: int) -> float:
@@ -538,7 +553,7 @@ def run_assign_section(ctx, reps: int = 5) -> dict:
     ref = O.assign_centers(sample, c, L)
     cpu_s = time.perf_counter() - t0
     same = bool(np.array_equal(ref, host[:20000]) and np.array_equal(out.cpu().numpy(), host))
-    alu_ops = 4 * L  # two-lane Myers: 7 LOP3 + 1 PRMT per step for two distances
+    alu_ops = sliced_ops_per_pair(L, 8)  # delta form, band half-width 3
     peaks, _ = measured_peaks()
     dev_s = min(ms) / 1e3
     alu_peak = torch.cuda.get_device_properties(0).multi_processor_count * 64 * float(
@@ -973,7 +988,8 @@ def run_ours(args, wl, rank, world, dist):
     alu_peak = props.multi_processor_count * 64 * sm_mhz * 1e6 / 1e12  # ALU pipe: 64 lanes/clk/SM
     int32_peak = props.multi_processor_count * 128 * sm_mhz * 1e6 / 1e12
     pair_avg_s = (pair_ms / max(pair_launches, 1)) / 1e3
-    alu_ops = pairs * sliced_ops_per_pair(L, d)
+    pair_kernel, ops_per_pair = build_pass_of(words, L, d)
+    alu_ops = pairs * ops_per_pair
     achieved = alu_ops / pair_avg_s / 1e12 if pair_launches else None
     conv_ops = pairs * 16 * L
     conv_achieved = conv_ops / pair_avg_s / 1e12 if pair_launches else None
@@ -983,7 +999,8 @@ def run_ours(args, wl, rank, world, dist):
     # count read + 4 B prefix written per (row, segment) cell a row uses (its
     # band's diagonal segment onwards), 24 B per row (degree, offset scan,
     # offset read)
-    cells = touched_cells(n, seg_width, segments)
+    # (prefix_pairs keeps no count cells)
+    cells = 0 if pair_kernel == "prefix_pairs" else touched_cells(n, seg_width, segments)
     comp_bytes = 12 * edges + 8 * cells + 24 * (n + 1)
     comp_avg_s = (comp_ms / max(comp_launches, 1)) / 1e3
     line = {
@@ -996,8 +1013,8 @@ def run_ours(args, wl, rank, world, dist):
         "e2e": e2e,
         "roofline": {"bound": "int32-alu-pipe", "achieved": achieved, "peak": alu_peak, "unit": "Tops/s",
                      "frac": (achieved / alu_peak) if achieved else None, "traffic": traffic,
-                     "kernel": "pair_levels", "kernel_ms_per_launch": pair_avg_s * 1e3,
-                     "work": f"{pairs} pair tests x {sliced_ops_per_pair(L, d):g} ALU-pipe ops (LOP3, 32 pair tests each) per pair "
+                     "kernel": pair_kernel, "kernel_ms_per_launch": pair_avg_s * 1e3,
+                     "work": f"{pairs} pair tests x {ops_per_pair:.4g} ALU-pipe ops (LOP3, 32 pair tests each) per pair "
                              f"test per launch",
                      "peak_source": f"{props.multi_processor_count} SMs x 64 ALU-pipe lanes/clk x {sm_mhz:.0f} MHz "
                                     f"max SM clock ({src} MEASURED_PEAKS sm_max_mhz)",
