@@ -11,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -53,8 +54,8 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     if not force:
         return LIB
     os.makedirs(BUILD_DIR, exist_ok=True)
-    objs = []
-    for src in sources():
+
+    def compile_one(src):
         obj = os.path.join(BUILD_DIR, os.path.basename(src) + ".o")
         cmd = [nvcc()] + ARCH + NVCC_FLAGS + ["-c", src, "-o", obj]
         if ptxas_info and src.endswith(".cu"):
@@ -62,7 +63,10 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
-        objs.append(obj)
+        return obj
+
+    with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        objs = list(pool.map(compile_one, sources()))
     tmp = LIB + ".tmp"
     cmd = [nvcc()] + ARCH + ["-shared", "-cudart", "static", "-o", tmp] + objs + ["-lpthread"]
     if verbose:
