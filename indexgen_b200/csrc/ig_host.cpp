@@ -280,6 +280,8 @@ class BucketGreedy {
                 if (t + 4 < nt)
                     rows_.prefetch(todel_[(size_t)t + 4]);
                 const int32_t i = todel_[(size_t)t];
+                if (deg[i] < 0)  // a list may name a vertex twice, or its own
+                    continue;
                 const int32_t *ri = rows_.get(i, bufi_.data());
                 const int64_t e = ap_[i + 1] - ap_[i];
                 for (int64_t k0 = 0; k0 < e; k0 += kChunk) {
