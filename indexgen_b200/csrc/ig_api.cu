@@ -319,7 +319,52 @@ ig_status make_jobs(Ctx *ctx, const int64_t *offsets, int32_t k, const int32_t *
     return IG_OK;
 }
 
+// The graph of jobs in `words` (host or device).  `finished`: the call returns
+// with the device done, as the public builds do; without it the exact copy of
+// the columns may still be under way on the context stream, in order with
+// whatever the library queues there next.
+ig_status build_words(ig_ctx *ctx, const uint32_t *words, int32_t n, int words_on_device,
+                      const std::vector<JobSpec> &jobs, bool finished, ig_graph **out)
+{
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    DeviceGuard dg(ctx->device);
+    if (!dg.ok)
+        return set_error(ctx, IG_ERR_CUDA, "cannot select the context's device");
+    ig_graph *g = new (std::nothrow) ig_graph();
+    if (!g)
+        return IG_ERR_OOM;
+    const uint32_t *d_words = nullptr;
+    ig_status s = stage_words(ctx, words, n, words_on_device, &d_words);
+    if (s == IG_OK)
+        s = build_batch(ctx, d_words, jobs, g);
+    if (s == IG_OK && finished) {
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess)
+            s = cuda_error(ctx, e, "column copy");
+    }
+    if (s != IG_OK) {
+        release_graph(g, true);
+        return s;
+    }
+    *out = g;
+    return IG_OK;
+}
+
 }  // namespace
+
+ig_status build_jobs(ig_ctx *ctx, const uint32_t *words, const int64_t *offsets, int32_t jobs, const int32_t *lens,
+                     const int32_t *min_eds, int words_on_device, bool finished, ig_graph **out)
+{
+    *out = nullptr;
+    std::vector<JobSpec> spec;
+    const ig_status s = make_jobs(ctx, offsets, jobs, lens, min_eds, spec);
+    if (s != IG_OK)
+        return s;
+    const int64_t total = jobs > 0 ? offsets[jobs] : 0;
+    if (total > 0 && !words)
+        return set_error(ctx, IG_ERR_INPUT, "words must be non-null");
+    return build_words(ctx, words, (int32_t)total, words_on_device, spec, finished, out);
+}
 
 // fetch_adjacency with the copy on the context's download stream: returns
 // once the copy is queued, followed by the host function `then(arg)` (run by
@@ -687,7 +732,7 @@ void build_requests(ig_ctx *ctx, const std::vector<SolveRequest *> &reqs)
             eds.push_back(r->min_ed);
         }
         ig_graph *g = nullptr;
-        s = ig_batch_build(ctx, words.data(), off.data(), (int32_t)reqs.size(), lens.data(), eds.data(), 0, &g);
+        s = build_jobs(ctx, words.data(), off.data(), (int32_t)reqs.size(), lens.data(), eds.data(), 0, false, &g);
         if (s == IG_OK) {
             auto hg = std::make_shared<HostGraph>();
             s = download_for_greedy(g, 1, *hg);
@@ -800,8 +845,8 @@ ig_status solve_groups(ig_ctx *ctx, const uint32_t *words, int words_on_device, 
         for (int j = lo; j <= hi; ++j)
             sub[(size_t)(j - lo)] = offsets[j] - offsets[lo];
         ig_graph *g = nullptr;
-        s = ig_batch_build(ctx, words + offsets[lo], sub.data(), hi - lo, lens + lo, min_eds + lo, words_on_device,
-                           &g);
+        s = build_jobs(ctx, words + offsets[lo], sub.data(), hi - lo, lens + lo, min_eds + lo, words_on_device, false,
+                       &g);
         const ig_status f = finish();  // the previous group's copy ran during this build
         if (s == IG_OK)
             s = f;
@@ -1070,23 +1115,7 @@ ig_status ig_graph_build(ig_ctx *ctx, const uint32_t *words, int32_t n, int len,
     *out = nullptr;
     if (ig::check_job(words, n, len) != IG_OK)
         return ig::set_error(ctx, IG_ERR_INPUT, "words must be non-null, n >= 0 and 1 <= len <= 16");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    ig::DeviceGuard dg(ctx->device);
-    if (!dg.ok)
-        return ig::set_error(ctx, IG_ERR_CUDA, "cannot select the context's device");
-    ig_graph *g = new (std::nothrow) ig_graph();
-    if (!g)
-        return IG_ERR_OOM;
-    const uint32_t *d_words = nullptr;
-    ig_status s = ig::stage_words(ctx, words, n, words_on_device, &d_words);
-    if (s == IG_OK)
-        s = ig::build_batch(ctx, d_words, {ig::JobSpec{0, n, len, min_ed}}, g);
-    if (s != IG_OK) {
-        ig::release_graph(g, true);
-        return s;
-    }
-    *out = g;
-    return IG_OK;
+    return ig::build_words(ctx, words, n, words_on_device, {ig::JobSpec{0, n, len, min_ed}}, true, out);
     IG_ABI_CATCH
 }
 
@@ -1166,15 +1195,6 @@ ig_status ig_graph_device_csr(const ig_graph *g, const int64_t **row_ptr, const 
     IG_ABI_TRY
     if (!g || !row_ptr || !cols)
         return IG_ERR_INPUT;
-    ig_graph *m = const_cast<ig_graph *>(g);
-    if (m->cols_pending) {
-        std::lock_guard<std::mutex> lk(g->ctx->mu);
-        ig::DeviceGuard dg(g->ctx->device);
-        const cudaError_t e = cudaStreamSynchronize(g->ctx->stream);
-        if (e != cudaSuccess)
-            return ig::cuda_error(g->ctx, e, "column copy");
-        m->cols_pending = false;
-    }
     *row_ptr = g->d_row_ptr;
     *cols = g->d_cols;
     return IG_OK;
@@ -1292,30 +1312,7 @@ ig_status ig_batch_build(ig_ctx *ctx, const uint32_t *words, const int64_t *offs
     if (!ctx || !out)
         return IG_ERR_INPUT;
     *out = nullptr;
-    std::vector<ig::JobSpec> spec;
-    ig_status s = ig::make_jobs(ctx, offsets, jobs, lens, min_eds, spec);
-    if (s != IG_OK)
-        return s;
-    const int64_t total = jobs > 0 ? offsets[jobs] : 0;
-    if (total > 0 && !words)
-        return ig::set_error(ctx, IG_ERR_INPUT, "words must be non-null");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    ig::DeviceGuard dg(ctx->device);
-    if (!dg.ok)
-        return ig::set_error(ctx, IG_ERR_CUDA, "cannot select the context's device");
-    ig_graph *g = new (std::nothrow) ig_graph();
-    if (!g)
-        return IG_ERR_OOM;
-    const uint32_t *d_words = nullptr;
-    s = ig::stage_words(ctx, words, (int32_t)total, words_on_device, &d_words);
-    if (s == IG_OK)
-        s = ig::build_batch(ctx, d_words, spec, g);
-    if (s != IG_OK) {
-        ig::release_graph(g, true);
-        return s;
-    }
-    *out = g;
-    return IG_OK;
+    return ig::build_jobs(ctx, words, offsets, jobs, lens, min_eds, words_on_device, true, out);
     IG_ABI_CATCH
 }
 
@@ -1471,7 +1468,9 @@ ig_status ig_solve(ig_ctx *ctx, const uint32_t *words, int32_t n, int len, int m
     {
         std::lock_guard<std::mutex> slot(ctx->solve_slot);
         ig_graph *g = nullptr;
-        ig_status s = ig_graph_build(ctx, words, n, len, min_ed, 0, &g);
+        if (ig::check_job(words, n, len) != IG_OK)
+            return ig::set_error(ctx, IG_ERR_INPUT, "words must be non-null, n >= 0 and 1 <= len <= 16");
+        ig_status s = ig::build_words(ctx, words, n, 0, {ig::JobSpec{0, n, len, min_ed}}, false, &g);
         if (s != IG_OK)
             return s;
         if (edges)

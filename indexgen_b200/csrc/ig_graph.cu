@@ -1875,13 +1875,11 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         return IG_OK;
     }
     IG_CUDA(dev_malloc(ctx, (void **)&g->d_cols, std::max<size_t>((size_t)total, 1) * sizeof(int32_t), st));
-    if (total > 0) {
-        // the copy is in order with everything the library does on the stream;
-        // only a caller that takes the raw pointers has to see it finished
+    if (total > 0)
+        // in order with everything the library does on the stream; the public
+        // builds wait for it
         IG_CUDA(cudaMemcpyAsync(g->d_cols, ctx->cols_ws.ptr, (size_t)total * sizeof(int32_t), cudaMemcpyDeviceToDevice,
                                 st));
-        g->cols_pending = true;
-    }
     return IG_OK;
 }
 

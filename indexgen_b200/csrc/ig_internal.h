@@ -209,7 +209,6 @@ struct Graph {
     std::vector<int32_t> job_seg_shift, job_nseg;  // pair-pass tiling per job (0 when not built here)
     int64_t *d_row_ptr = nullptr;       // [n+1]
     int32_t *d_cols = nullptr;          // [edges], global column ids
-    std::atomic<bool> cols_pending{false};  // d_cols is still being copied on the context stream
     // host copies, filled on first use
     std::vector<int64_t> h_row_ptr;
     std::vector<int32_t> h_cols;
@@ -236,7 +235,8 @@ struct PairPlan {
 // Plan for a job of n words that should yield about `target_items` items.
 PairPlan make_plan(int32_t n, long long target_items);
 
-// Device pipeline stages (ig_graph.cu).  Jobs index into d_words.
+// Device pipeline stages (ig_graph.cu).  Jobs index into d_words.  build_batch
+// may leave the copy of the columns under way on the context stream.
 ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, Graph *g);
 ig_status count_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, int64_t *edges);
 // Threshold class of (len, min_ed), IG_LANES_* (ig_graph.cu).
@@ -347,6 +347,10 @@ struct PooledGreedyScope {
     bool on_;
 };
 
+// ig_batch_build; with `finished` false, without the wait for the columns
+// (ig_api.cu).
+ig_status build_jobs(ig_ctx *ctx, const uint32_t *words, const int64_t *offsets, int32_t jobs, const int32_t *lens,
+                     const int32_t *min_eds, int words_on_device, bool finished, ig_graph **out);
 // Builds the jobs (words [offsets[j], offsets[j+1]), host or device pointer)
 // in up to eight groups and runs their greedies on host_threads threads as
 // each group arrives; job j's selection goes to order + offsets[j], its size

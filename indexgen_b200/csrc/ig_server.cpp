@@ -252,7 +252,7 @@ void ig_server::schedule_loop()
         }
         ig_graph *g = nullptr;
         if (s == IG_OK)
-            s = ig_batch_build(ctx, words.data(), off.data(), (int32_t)batch.size(), lens.data(), eds.data(), 0, &g);
+            s = ig::build_jobs(ctx, words.data(), off.data(), (int32_t)batch.size(), lens.data(), eds.data(), 0, false, &g);
         finish_pending();  // the previous batch's copy ran during this build
         if ((s == IG_ERR_OOM || s == IG_ERR_CAPACITY) && batch.size() > 1) {
             // the merged build failed where each job alone may not: they go
