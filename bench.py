@@ -352,15 +352,16 @@ def sliced_ops_per_pair(L: int, d: int) -> float:
     return level_ops(L, k, (0, L))[0] / 32
 
 
-PREFIX_MIN_WORDS, PREFIX_MIN_LEN, PREFIX_LONG_WORDS = 32768, 10, 131072  # ig_internal.h
+PREFIX_LONG_WORDS = 131072  # kPrefixLongWords, ig_internal.h
 
 
-def build_pass_of(words, L: int, d: int):
+def build_pass_of(words, L: int, d: int, shared_prefixes: bool):
     """(pair kernel, LOP3 operations per pair test) of a lone build of these
-    words: with shared prefixes (ig_prefix.cu) the levels of the first D1 and D2
-    characters run once per distinct prefix, not once per word."""
+    words: with shared prefixes (ig_prefix.cu; the graph's tiling tells) the
+    levels of the first D1 and D2 characters run once per distinct prefix, not
+    once per word."""
     n = len(words)
-    if n < PREFIX_MIN_WORDS or L < PREFIX_MIN_LEN or not 3 <= d <= 5 or d >= L // 2:
+    if not shared_prefixes:
         return ("pair_levels" if d <= 5 else "pair_deltas"), sliced_ops_per_pair(L, d)
     d2 = 8 if n >= PREFIX_LONG_WORDS else 7
     d1 = d2 - 2
@@ -988,7 +989,7 @@ def run_ours(args, wl, rank, world, dist):
     alu_peak = props.multi_processor_count * 64 * sm_mhz * 1e6 / 1e12  # ALU pipe: 64 lanes/clk/SM
     int32_peak = props.multi_processor_count * 128 * sm_mhz * 1e6 / 1e12
     pair_avg_s = (pair_ms / max(pair_launches, 1)) / 1e3
-    pair_kernel, ops_per_pair = build_pass_of(words, L, d)
+    pair_kernel, ops_per_pair = build_pass_of(words, L, d, seg_width > 0 and segments == 0)
     alu_ops = pairs * ops_per_pair
     achieved = alu_ops / pair_avg_s / 1e12 if pair_launches else None
     conv_ops = pairs * 16 * L

@@ -237,8 +237,10 @@ ig_status ig_graph_job_count(const ig_graph *g, int32_t *jobs);
 ig_status ig_graph_job_stats(const ig_graph *g, int32_t job, int64_t *first_word, int32_t *n, int64_t *edges);
 /* Tiling the pair pass used for job j: column segments of segment_width
  * columns (a power of two, at most 65,536) and their number; each (row,
- * segment) pair had one count cell.  Zero for jobs without pair tests and for
- * graphs read from a file.  The replacement of the reference's fixed
+ * segment) pair had one count cell.  A lone large sparse job whose shared
+ * prefixes ran once has no segments and no count cells: segments is 0 and
+ * segment_width the width of its column blocks.  Both are zero for jobs
+ * without pair tests and for graphs read from a file.  The replacement of the reference's fixed
  * 16384 x 16384 tiles (src/cuda_edit_distance.py:380-390). */
 ig_status ig_graph_job_tiling(const ig_graph *g, int32_t job, int32_t *segment_width, int32_t *segments);
 /* Greedy of every job on host_threads host threads (0 = all cores), largest

@@ -1289,7 +1289,9 @@ ig_status ig_graph_job_tiling(const ig_graph *g, int32_t job, int32_t *segment_w
         return IG_ERR_INPUT;
     const bool known = (size_t)job < g->job_nseg.size();
     if (segment_width)
-        *segment_width = known && g->job_nseg[(size_t)job] > 0 ? 1 << g->job_seg_shift[(size_t)job] : 0;
+        *segment_width = g->shared_prefixes                        ? ig::kPrefixBlockCols
+                         : known && g->job_nseg[(size_t)job] > 0 ? 1 << g->job_seg_shift[(size_t)job]
+                                                                 : 0;
     if (segments)
         *segments = known ? g->job_nseg[(size_t)job] : 0;
     return IG_OK;

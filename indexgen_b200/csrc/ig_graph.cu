@@ -1790,10 +1790,6 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
     g->job_edge_off.assign(jobs.size() + 1, 0);
     g->job_seg_shift.clear();
     g->job_nseg.clear();
-    for (const JobDesc &d : B.desc) {
-        g->job_seg_shift.push_back(d.seg_shift);
-        g->job_nseg.push_back(d.nseg);
-    }
     IG_CUDA(dev_malloc(ctx, (void **)&g->d_row_ptr, ((size_t)n + 1) * sizeof(int64_t), st));
     if (B.items == 0) {
         IG_CUDA(cudaMemsetAsync(g->d_row_ptr, 0, ((size_t)n + 1) * sizeof(int64_t), st));
@@ -1862,6 +1858,12 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         }
     }
     g->edges = (int64_t)total;
+    g->shared_prefixes = prefix;
+    if (!prefix)
+        for (const JobDesc &d : B.desc) {
+            g->job_seg_shift.push_back(d.seg_shift);
+            g->job_nseg.push_back(d.nseg);
+        }
     const int njobs = (int)B.desc.size();
     if (g->job_edge_off[(size_t)njobs] != (int64_t)total)
         return set_error(ctx, IG_ERR_STATE, "row offsets disagree with the edge count");

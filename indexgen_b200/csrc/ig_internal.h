@@ -207,6 +207,7 @@ struct Graph {
     std::vector<JobSpec> jobs;          // one entry for a single-job graph
     std::vector<int64_t> job_edge_off;  // [jobs+1] row_ptr at job boundaries
     std::vector<int32_t> job_seg_shift, job_nseg;  // pair-pass tiling per job (0 when not built here)
+    bool shared_prefixes = false;       // built by prefix_pass: column blocks of kPrefixBlockCols, no segments
     int64_t *d_row_ptr = nullptr;       // [n+1]
     int32_t *d_cols = nullptr;          // [edges], global column ids
     // host copies, filled on first use
@@ -255,6 +256,7 @@ ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<Job
 // upper CSR; *slots > record capacity or *hits > col_cap: void, as for the
 // general pass.
 constexpr int kPrefixMinLen = 10;
+constexpr int kPrefixBlockCols = 2048;  // columns a work item tests its rows against
 // From here on it wins at every length and threshold it takes: a build of
 // 28,000 words took 137 us against 138 at L = 13, k = 2 and 261 against 276 at
 // L = 16, k = 4, one of 36,000 words 166 against 195 and 358 against 420;

@@ -57,6 +57,7 @@ using slice::Words2;
 constexpr int kWarps = 1;                        // warps of a CTA
 constexpr int kWarpCols = 2048;                  // columns of a warp
 constexpr int kBlockCols = kWarps * kWarpCols;   // columns of a CTA
+static_assert(kBlockCols == kPrefixBlockCols, "the tiling that a graph reports");
 constexpr int kTileRows = 16;                    // rows per staged tile
 constexpr int kRowBytes = 64;                    // a row record: 16 table offsets
 constexpr int kPosBytes = 1024;                  // table bytes per position: 4 characters x 32 lanes x 2 words

@@ -248,7 +248,8 @@ class ConflictGraph:
         return int(f.value), int(n.value), int(e.value)
 
     def job_tiling(self, job: int = 0):
-        """(segment width, segments) of the pair pass that built one job."""
+        """(segment width, segments) of the pair pass that built one job; no
+        segments but a width: its shared prefixes ran once, in column blocks."""
         w = ctypes.c_int32()
         k = ctypes.c_int32()
         check(lib().ig_graph_job_tiling(self.handle, int(job), ctypes.byref(w), ctypes.byref(k)),
