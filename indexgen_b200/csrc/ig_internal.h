@@ -257,9 +257,9 @@ ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<Job
 // general pass.
 constexpr int kPrefixMinLen = 10;
 constexpr int kPrefixBlockCols = 2048;  // columns a work item tests its rows against
-// From here on it wins at every length and threshold it takes: a build of
-// 28,000 words took 137 us against 138 at L = 13, k = 2 and 261 against 276 at
-// L = 16, k = 4, one of 36,000 words 166 against 195 and 358 against 420;
+// From here on its pair pass wins at every length and threshold it takes: a
+// build of 28,000 words took 137 us against 138 at L = 13, k = 2 and 261 against
+// 276 at L = 16, k = 4, one of 36,000 words 166 against 195 and 358 against 420;
 // with 20,000 words the general pass is faster.
 constexpr int32_t kPrefixMinWords = 32768;
 constexpr int32_t kPrefixLongWords = 131072;  // prefixes of 8 characters instead of 7
@@ -269,6 +269,9 @@ struct PrefixOut {
     unsigned long long col_cap = 0;
 };
 bool prefix_job(const JobSpec &j);
+// Whether a build of the job should run it: its columns come out unsorted,
+// which costs more the more of them a word has.
+bool prefix_build(const JobSpec &j);
 ig_status prefix_pass(Ctx *ctx, const uint32_t *d_words, const JobSpec &job, const PrefixOut *out,
                       unsigned long long *slots, unsigned long long *hits, int64_t *bounds);
 // Status word of a finished pair pass as a status with its message, and

@@ -730,6 +730,33 @@ bool prefix_job(const JobSpec &j)
     return j.n >= kPrefixMinWords && j.len >= kPrefixMinLen && t.L == j.len && t.levels && t.k >= 2;
 }
 
+// The saving grows with the pair tests (0.06 to 0.2 ns each), the cost of
+// degrees, placing and sorting with the edges: 15 to 30 ps each up to about 130
+// edges a word, 45 at 156, 65 to 135 at 220, where half of the rows are too
+// long for a warp's registers.  What decides is the share of pairs that are
+// edges, for uniform words a matter of length and threshold, and the word
+// count.  Whole builds of uniform words on a B200, this pass against the general
+// one, ms:
+//   L = 10, k = 2  400,000 6.5 / 11.6   800,000 46.7 / 45.7
+//   L = 10, k = 3   33,000 0.34 / 0.25   60,000 1.04 / 0.62
+//   L = 11, k = 3   50,000 0.40 / 0.45  130,000 2.07 / 2.26  145,000 2.87 / 2.83  160,000 3.71 / 3.47
+//   L = 12, k = 3  300,000 6.7 / 11.6   600,000 37.3 / 45.6
+//   L = 12, k = 4   33,000 0.41 / 0.34   60,000 1.30 / 0.95
+//   L = 13, k = 4   60,000 0.82 / 0.90  209,000 9.65 / 10.08
+//   L = 14, k = 4  300,000 13.2 / 20.6  500,000 41.4 / 56.3
+// So: never at (10, 3) and (12, 4), up to 140,000 and 750,000 words at (11, 3)
+// and (10, 2), elsewhere up to 256 edges a word (densities of 8 x 10^8 uniform
+// pairs per length and threshold); jobs of editDist >= L/2 keep hit words.
+bool prefix_build(const JobSpec &j)
+{
+    constexpr int32_t any = kMaxJobWords;
+    static const int32_t most[IG_MAX_LEN - kPrefixMinLen + 1][3] = {  // by length and k = 2..4
+        {750000, 0, 0},        {2988000, 140000, 0},   {10026000, 705000, 0}, {any, 2136000, 206000},
+        {any, 6616000, 572000}, {any, any, 1638000},    {any, any, 4776000},
+    };
+    return prefix_job(j) && j.n <= most[j.len - kPrefixMinLen][j.min_ed - 3];
+}
+
 ig_status prefix_pass(Ctx *ctx, const uint32_t *d_words, const JobSpec &job, const PrefixOut *out,
                       unsigned long long *slots, unsigned long long *hits, int64_t *bounds)
 {
