@@ -1774,18 +1774,20 @@ ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<Job
 // 150 (500 a word) 4.7 against 4.0 (k = 2) to 7.6 (k = 4).
 constexpr unsigned long long kPrefixMaxDegree = 320;
 
-ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, Graph *g)
+namespace {
+
+// build_batch with hit words in at most bits_limit bytes; *hit_words: whether
+// any job keeps them.
+ig_status build_planned(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, size_t bits_limit,
+                        Graph *g, bool *hit_words)
 {
     cudaStream_t st = ctx->stream;
-    ig_status s = check_jobs(ctx, jobs);
-    if (s == IG_OK)
-        s = autotune_jobs(ctx, d_words, jobs);
-    if (s != IG_OK)
-        return s;
+    ig_status s = IG_OK;
     const int grid = pair_grid(ctx);
     BatchLayout B;
-    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, std::max(ctx->records.bytes, kBitsRoom), B))
+    if (!plan_batch(jobs, grid, ctx->pair_grid_levels, ctx->items_per_cta, bits_limit, B))
         return set_error(ctx, IG_ERR_CAPACITY, "batch too large for one launch");
+    *hit_words = B.bits > 0;
     const int32_t n = (int32_t)B.rows;
     g->ctx = ctx;
     g->n = n;
@@ -1793,7 +1795,8 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
     g->job_edge_off.assign(jobs.size() + 1, 0);
     g->job_seg_shift.clear();
     g->job_nseg.clear();
-    IG_CUDA(dev_malloc(ctx, (void **)&g->d_row_ptr, ((size_t)n + 1) * sizeof(int64_t), st));
+    if (!g->d_row_ptr)
+        IG_CUDA(dev_malloc(ctx, (void **)&g->d_row_ptr, ((size_t)n + 1) * sizeof(int64_t), st));
     if (B.items == 0) {
         IG_CUDA(cudaMemsetAsync(g->d_row_ptr, 0, ((size_t)n + 1) * sizeof(int64_t), st));
         IG_CUDA(cudaStreamSynchronize(st));
@@ -1888,6 +1891,32 @@ ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSp
         IG_CUDA(cudaMemcpyAsync(g->d_cols, ctx->cols_ws.ptr, (size_t)total * sizeof(int32_t), cudaMemcpyDeviceToDevice,
                                 st));
     return IG_OK;
+}
+
+}  // namespace
+
+ig_status build_batch(Ctx *ctx, const uint32_t *d_words, const std::vector<JobSpec> &jobs, Graph *g)
+{
+    ig_status s = check_jobs(ctx, jobs);
+    if (s == IG_OK)
+        s = autotune_jobs(ctx, d_words, jobs);
+    if (s != IG_OK)
+        return s;
+    bool hit_words = false;
+    s = build_planned(ctx, d_words, jobs, std::max(ctx->records.bytes, kBitsRoom), g, &hit_words);
+    if (s != IG_ERR_OOM || !hit_words)
+        return s;
+    // Hit words take n^2/16 bytes whatever the edges are, and the columns get
+    // room to match: where that does not fit, records may.
+    for (DevBuf *b : {&ctx->records, &ctx->cols_ws}) {
+        if (b->ptr)
+            cudaFreeAsync(b->ptr, ctx->stream);
+        b->ptr = nullptr;
+        b->bytes = 0;
+    }
+    ctx->col_room = 0;
+    IG_CUDA(cudaStreamSynchronize(ctx->stream));
+    return build_planned(ctx, d_words, jobs, 0, g, &hit_words);
 }
 
 }  // namespace ig
