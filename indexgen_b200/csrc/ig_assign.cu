@@ -9,14 +9,14 @@
 // running minimum in registers; only the N int32 assignments leave the device.
 // Ties go to the lowest centre index, as np.argmin's first occurrence does.
 //
-// Two kernels.  assign_sliced (9 centres or more): one word per thread against
-// 64 centres per step, bit-sliced (ig_slice.cuh), centre tables staged in
-// shared memory, 2,048 per pass.  assign_kernel (fewer, where most of a word's
-// bits would stand for no centre): centres are the Myers patterns (their Peq
-// pools in shared memory), words the texts: each thread holds the selector
-// stream of two words (two 16-bit lanes, L <= 15) or one (L = 16) in registers
-// and walks all centres with the full Myers recurrence of ig_myers.cuh,
-// reading the exact distance at the end.
+// Two kernels.  assign_sliced (from 9 to 13 centres on, by length and word
+// count): one word per thread against 64 centres per step, bit-sliced
+// (ig_slice.cuh), centre tables staged in shared memory, 2,048 per pass.
+// assign_kernel (fewer, where most of a word's bits would stand for no centre):
+// centres are the Myers patterns (their Peq pools in shared memory), words the
+// texts: each thread holds the selector stream of two words (two 16-bit lanes,
+// L <= 15) or one (L = 16) in registers and walks all centres with the full
+// Myers recurrence of ig_myers.cuh, reading the exact distance at the end.
 #include <algorithm>
 #include <climits>
 
@@ -287,9 +287,28 @@ __global__ void __launch_bounds__(kAssignThreads, 3) assign_sliced(const uint32_
 // L = 7.
 //
 // A word costs the same for 1 to 32 centres, so below some count assign_kernel
-// wins: 1,000,000 words, k = 8 against k = 9, took 46 against 41 us at L = 10,
-// 53 against 54 at L = 13 and 101 against 69 at L = 16.
-constexpr int kSlicedMinCentres = 9;
+// wins; later for fewer words, whose last wave of persistent blocks is emptier.
+// assign_kernel / assign_sliced, us:
+//            300,000 words               1,000,000 words
+//   L = 10   k = 9 26.3 / 25.4           k = 9 47.9 / 40.0
+//   L = 11   k = 9 27.7 / 29.0           k = 9 51.6 / 45.2
+//            k = 11 29.4 / 29.0
+//   L = 12   k = 9 28.6 / 27.8           k = 9 54.1 / 56.4, k = 10 57.5 / 49.4
+//   L = 13   k = 9 28.9 / 29.6           k = 9 55.1 / 53.1
+//            k = 10 30.1 / 29.6
+//   L = 14   k = 9 29.8 / 33.0           k = 9 58.5 / 62.4
+//            k = 11 32.1 / 30.9          k = 11 66.3 / 57.4
+//   L = 15   k = 9 30.5 / 33.3           k = 9 61.3 / 63.9
+//            k = 12 34.4 / 36.7          k = 12 73.8 / 67.6
+//            k = 13 35.7 / 34.2
+//   L = 16   k = 9 45.6 / 33.9           k = 9 110 / 67
+constexpr long long kManyWords = 1 << 19;
+
+__host__ __device__ constexpr int sliced_from(int L, bool many)
+{
+    return L == 11 ? (many ? 9 : 11) : L == 12 ? 10 : L == 13 ? (many ? 9 : 10) : L == 14 ? (many ? 10 : 11)
+           : L == 15 ? (many ? 12 : 13) : 9;
+}
 
 __host__ __device__ constexpr int min_centres(int L, int W)
 {
@@ -305,8 +324,8 @@ void launch_sliced(Ctx *ctx, const uint32_t *words, long long n, const uint32_t 
     assign_sliced<L, W><<<(unsigned)blocks, kAssignThreads, 0, ctx->stream>>>(words, n, centres, k, out, 1u);
 }
 
-// The narrowest band whose repeats are rare; lengths whose 9 centres always
-// suffice for W = 3 or 4 have no wider variant.
+// The narrowest band whose repeats are rare; lengths whose fewest centres
+// always suffice for W = 3 or 4 have no wider variant.
 template <int L>
 void launch_sliced_len(Ctx *ctx, const uint32_t *words, long long n, const uint32_t *centres, int k, int32_t *out)
 {
@@ -314,12 +333,12 @@ void launch_sliced_len(Ctx *ctx, const uint32_t *words, long long n, const uint3
         launch_sliced<L, 3>(ctx, words, n, centres, k, out);
         return;
     }
-    if constexpr (min_centres(L, 3) > kSlicedMinCentres) {
+    if constexpr (min_centres(L, 3) > sliced_from(L, true)) {
         if (k >= min_centres(L, 4)) {
             launch_sliced<L, 4>(ctx, words, n, centres, k, out);
             return;
         }
-        if constexpr (min_centres(L, 4) > kSlicedMinCentres)
+        if constexpr (min_centres(L, 4) > sliced_from(L, true))
             launch_sliced<L, 5>(ctx, words, n, centres, k, out);
     }
 }
@@ -331,7 +350,7 @@ void launch_assign_len(Ctx *ctx, int grid, const uint32_t *words, long long n, c
                        int32_t *out)
 {
     const cudaStream_t st = ctx->stream;
-    if (k >= kSlicedMinCentres) {
+    if (k >= sliced_from(L, n >= kManyWords)) {
         launch_sliced_len<L>(ctx, words, n, centres, k, out);
         return;
     }
