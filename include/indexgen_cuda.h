@@ -65,8 +65,9 @@ int64_t ig_ctx_launches(const ig_ctx *ctx);
  * (row offsets + scatter into CSR), IG_PHASE_PREP (column units), and the
  * parts of IG_PHASE_COMPACT: IG_PHASE_PREFIX (per-row prefix of the segment
  * counts and, in the same kernel, the row offsets), IG_PHASE_SCAN (no longer
- * apart: 0 launches), IG_PHASE_SCATTER (records or hit words into columns).  ig_ctx_phase_time returns the accumulated
- * milliseconds and launch count since profiling was last enabled. */
+ * apart: 0 launches), IG_PHASE_SCATTER (records or hit words into columns).
+ * ig_ctx_phase_time returns the accumulated milliseconds and launch count
+ * since profiling was last enabled. */
 #define IG_PHASE_PAIRS 0
 #define IG_PHASE_COMPACT 1
 #define IG_PHASE_PREP 2
@@ -97,7 +98,9 @@ int ig_lane_form(int len, int min_ed);
  * (6, 12, 24, 48, 96 items per CTA; CUDA events on the context's stream,
  * best of two after a warm-up) and keeps the fastest for the job's lane
  * form; *items_per_cta (optional) = the choice.  Results never depend on
- * the split.  With autotuning on (the default) a context tunes each lane
+ * the split, and a lone build whose shared prefixes run once
+ * (ig_graph_job_tiling) does not use it: the choice then serves batches and
+ * smaller jobs.  With autotuning on (the default) a context tunes each lane
  * form by itself on the first batch build (two or more jobs) whose
  * candidates cut differently: on the batch's jobs of that form, or on a
  * 131,072-word sample of the largest of them when they hold more than 2^33
@@ -162,11 +165,12 @@ ig_status ig_ctx_set_coalescing(ig_ctx *ctx, int enable);
 ig_status ig_ctx_coalesce_stats(ig_ctx *ctx, int64_t *batches, int64_t *requests);
 
 /* ---- CUDA graphs of the batch pipeline ---------------------------------- */
-/* Each build (single job or batch) is one CUDA graph launch on the
- * context's stream -- job table upload, selector streams, the persistent pair
- * kernel(s), then the compaction into CSR (row offsets, scan, scatter, job
- * bounds) and the status readback -- with one host wait at the end.  A build
- * whose arguments equal the cached graph's relaunches it; otherwise the calls
+/* A build (single job or batch) is one CUDA graph launch on the context's
+ * stream -- column units, the persistent pair kernel(s), then the compaction
+ * into CSR (row offsets; records or hit words into columns), whose last
+ * kernel reports the status and the job bounds -- and a host wait.  (A lone
+ * large sparse job whose shared prefixes run once queues its kernels directly
+ * and counts no graph launch.)  A build whose arguments equal the cached graph's relaunches it; otherwise the calls
  * are captured and applied to the cached executable graph with
  * cudaGraphExecUpdate, so a batch of a known shape costs no instantiation.
  * On by default; per-phase timing (ig_ctx_set_profiling) runs the same calls
@@ -274,7 +278,7 @@ typedef struct ig_server_opts {
     int max_batch_jobs;        /* jobs per launch (0 = 256)                       */
     int order_threads;         /* neighbour order (0 or 1 = canonical sorted)     */
     int reserved;
-    int64_t max_batch_pairs;   /* pair tests per launch (0 = 2e10, ~0.1 s)        */
+    int64_t max_batch_pairs;   /* pair tests per launch (0 = 2e10, 5 to 10 ms)    */
     int64_t hbm_budget_bytes;  /* estimated HBM per launch (0 = half the free HBM) */
     int64_t pool_reserve_bytes; /* device memory taken into the context's stream-
                                  * ordered pool at start, so that the first large

@@ -684,8 +684,8 @@ std::shared_ptr<SolveCombiner> solve_combiner(Ctx *ctx)
 }
 
 // The waiting requests one coalesced build takes, in arrival order: the
-// first always, more while the batch stays within 2^36 pair tests (about
-// 0.1 s of device work) and 2^26 words; the rest wait for the next build.
+// first always, more while the batch stays within 2^36 pair tests (17 to 35 ms
+// of device work at editDist 4 and 5) and 2^26 words; the rest wait for the next build.
 void take_coalesced(std::vector<SolveRequest *> &pending, std::vector<SolveRequest *> &batch)
 {
     long double pairs = 0;
@@ -789,8 +789,8 @@ ig_status solve_groups(ig_ctx *ctx, const uint32_t *words, int words_on_device, 
     for (int32_t j = 0; j < jobs; ++j)
         total += (long double)(offsets[j + 1] - offsets[j]) * (offsets[j + 1] - offsets[j]);
     // a group costs a few hundred microseconds of host round trips besides
-    // its device work, so each one gets at least 2^30 pair tests (about
-    // 1.4 ms on nibble lanes): small batches stay one launch
+    // its device work, so each one gets at least 2^30 pair tests (0.3 ms at
+    // editDist 4, L = 12): small batches stay one launch
     const long double min_group = (long double)(1ull << 31);  // total counts n^2, not n(n-1)/2
     const int groups = (int)std::max<long double>(1, std::min<long double>({8.0L, (long double)jobs, total / min_group}));
     std::vector<int> cut{0};

@@ -619,7 +619,8 @@ __global__ void __launch_bounds__(kBandRows, 2) pair_deltas(PairArgs a) { pair_l
 // build went from 13 graph nodes to 5, and 2,000 words at L = 12, editDist 4
 // from 122 to 100 us, 19,999 at L = 13, editDist 7 from 378 to 346.
 //
-// Look-back: a block takes its number from a ticket, so every block before it
+// Look-back (decoupled look-back: Merrill and Garland, "Single-pass Parallel
+// Prefix Scan with Decoupled Look-back", 2016): a block takes its number from a ticket, so every block before it
 // is already running; it publishes its own degree sum, then adds up the
 // blocks before it from their published words, 32 at a time, until one holds
 // a complete prefix, and publishes its own.  A word is the sum in 62 bits
@@ -1281,10 +1282,11 @@ struct CompactOut {
     int32_t n = 0;
 };
 
-// One pass over a planned batch: job table upload, selector streams, the pair
-// kernel(s) and, for a build (`out` set), the compaction into out's CSR (row
-// offsets from the per-(row, segment) counts, scan, scatter of the records,
-// job bounds) -- queued as ONE graph launch with one host wait at the end.
+// One pass over a planned batch: column units (with the job table, uploaded
+// before them when it is long), the pair kernel(s) and, for a build (`out`
+// set), the compaction into out's CSR (row offsets from the per-(row, segment)
+// counts, records or hit words into columns, job bounds) -- queued as ONE graph
+// launch with one host wait at the end.
 // *slots = record slots handed out (>= *hits; the pass is complete iff they
 // fit the record buffer -- otherwise its CSR is void and the caller grows the
 // buffer and reruns), *hits = edges; bounds (build only) = row_ptr at the
@@ -1751,8 +1753,8 @@ ig_status autotune_jobs(Ctx *ctx, const uint32_t *d_words, const std::vector<Job
             }
         if (sub.empty())
             continue;
-        // Time the real jobs when a pass is short (<= 2^33 pair tests, about
-        // 10 ms on nibble lanes); otherwise the first 131,072 words of the
+        // Time the real jobs when a pass is short (<= 2^33 pair tests, 2 to 4 ms
+        // at editDist 4 and 5); otherwise the first 131,072 words of the
         // largest job stand in for them.
         if (pairs > (long double)(1ull << 33)) {
             JobSpec one = sub[largest];

@@ -151,9 +151,9 @@ struct Ctx {
     int64_t phase_launches[kPhases] = {};
     bool phase_pending[kPhases] = {};
     std::shared_ptr<PinnedPool> pinned = std::make_shared<PinnedPool>();
-    // CUDA graphs of the batch pipeline: [0] a build pass (job table upload,
-    // selector streams, pair kernels, row offsets, scan, scatter into CSR,
-    // job bounds, readback), [1] a count-only pass.  A pass whose arguments
+    // CUDA graphs of the batch pipeline: [0] a build pass (column units, pair
+    // kernels, row offsets, records or hit words into columns, report), [1] a
+    // count-only pass.  A pass whose arguments
     // equal the cached graph's relaunches it; otherwise it is captured and
     // applied to the cached executable graph with cudaGraphExecUpdate (a new
     // instantiation only when the topology changed).

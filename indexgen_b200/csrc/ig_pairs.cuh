@@ -126,7 +126,7 @@ __device__ __forceinline__ void warp_count_prefix(uint32_t cnt, int lane, unsign
     pre = incl - cnt;
 }
 
-// Words of a scan by decoupled look-back: a block's word is a sum in 62 bits
+// Words of a scan by decoupled look-back (Merrill and Garland, 2016): a block's word is a sum in 62 bits
 // under two bits saying what it is (0 nothing, 1 the block's own sum, 2 the
 // prefix up to and including the block).
 constexpr unsigned long long kOwnSum = 1ull << 62, kPrefixSum = 2ull << 62, kSumMask = (1ull << 62) - 1;

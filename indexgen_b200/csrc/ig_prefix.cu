@@ -540,7 +540,7 @@ __global__ void place_columns(const uint2 *__restrict__ rec, const unsigned long
     }
 }
 
-// Ascending bitonic sort of 32 E values, value e * 32 + lane in v[e].
+// Ascending bitonic sort (Batcher, 1968) of 32 E values, value e * 32 + lane in v[e].
 template <int E>
 __device__ __forceinline__ void warp_sort(int32_t (&v)[E], int lane)
 {

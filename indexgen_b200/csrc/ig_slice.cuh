@@ -220,7 +220,8 @@ struct Planes {
     uint32_t p[5];
 };
 
-// Carry-save counter.  Level l keeps one or two words of weight 2^l; a third
+// Carry-save counter (a column of full adders per bit weight, as in Wallace's
+// multiplier, 1964).  Level l keeps one or two words of weight 2^l; a third
 // goes through a full adder, whose carry arrives at the next level.  Which of
 // these a word meets depends only on how many arrived before it, so with the
 // row loop unrolled it is all known at compile time.
